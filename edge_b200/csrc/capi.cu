@@ -12,6 +12,7 @@
 #include "kernel_set.h"
 #include "kernels.cuh"
 #include "layout.cuh"
+#include "step_coef.cuh"
 
 namespace edge_b200 {
 KernelSet *makeKernelSet_o2(int, int, int, int);
@@ -182,19 +183,20 @@ __global__ void kBuildFsChar(const double *fsE, const int32_t *elFaEl, const uin
   }
 }
 
-// halo exchange: blocks [9][R][GF] of face slots (element * 4 + face) to / from a packed buffer,
-// 16 bytes per thread; slots outside the face buffer are skipped
-__global__ void kFacePack(uint4 *face, uint4 *buf, const int32_t *slots, int n, int64_t blk16, int64_t nSlots,
-                          bool pack) {
+// halo exchange: blocks of blk16 x 16 bytes of face slots (element * 4 + face) to / from a packed
+// buffer with stride16 x 16 bytes per slot, 16 bytes per thread; slots outside the face buffer are
+// skipped
+__global__ void kFacePack(uint4 *face, uint4 *buf, const int32_t *slots, int n, int64_t blk16, int64_t stride16,
+                          int64_t nSlots, bool pack) {
   const int64_t total = (int64_t)n * blk16;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t k = i / blk16, w = i % blk16;
     const int64_t sl = slots[k];
     if (sl < 0 || sl >= nSlots) continue;
     if (pack)
-      buf[i] = face[sl * blk16 + w];
+      buf[k * stride16 + w] = face[sl * blk16 + w];
     else
-      face[sl * blk16 + w] = buf[i];
+      face[sl * blk16 + w] = buf[k * stride16 + w];
   }
 }
 
@@ -304,14 +306,21 @@ struct edge_b200_ctx {
   bool fsLRChar = false;      // fsLR holds the characteristic factors of the pairs
   DevBuf charBad;             // device counter of the factor build's rank check
   bool charRejected = false;  // some face's pair is not of rank 3 (until the element data changes)
-  // fused GTS steps (pre-mixing configurations, no halo): within one multi-step call each local
-  // step also runs the previous step's neighbour step, so the face projections alternate between
-  // two buffers (faceCur holds the last written); the last step's neighbour step runs on its own at
+  // strong-form GTS steps (step.cuh): coefficients and gather table, rebuilt before the next GTS step
+  // after the mesh or the element data changed; flux solvers that are not of rank 3 in that form
+  // keep the context on the weak-form kernels until the data change again
+  DevBuf fac, gath, stepBad;
+  bool stepStale = true, stepRejected = false;
+  bool strong() const { return ks->strongSupported() && !stepStale && !stepRejected; }
+  // the face buffer ([nEl][4][9][R][GF]) then holds the characteristics the elements write for their
+  // neighbours ([nEl][4][3][R][GF], two of them, alternating with the steps: outCur holds the last
+  // written) and those they keep. Without halo parts, the steps of one multi-step call are fused:
+  // each step's surface integrals run in the next step's kernel, and the last one's on their own at
   // the end of the call (flush), so between calls nothing is pending
-  DevBuf faceAlt;
-  int faceCur = 0;
+  int outCur = 0;
   bool pending = false, fusedOn = true;
-  void *faceBuf(int i) const { return i ? faceAlt.p : face; }
+  char *faceThird(int i) const { return static_cast<char *>(face) + i * (faceCount() / 3 * realSize); }
+  void *outBuf(int i) const { return faceThird(i); }
   // sources
   SrcArgs src{};
   DevBuf srcMem[10];
@@ -404,6 +413,8 @@ struct edge_b200_ctx {
   size_t dofsCount() const { return (size_t)nEl * 9 * cfg.n_runs * GB; }
   size_t dofsACount() const { return (size_t)nEl * cfg.n_rms * 6 * cfg.n_runs * GB; }
   size_t faceCount() const { return (size_t)nEl * 4 * 9 * cfg.n_runs * GF; }
+  // the last third of the face buffer takes the own characteristics of whole element groups (32 lanes)
+  size_t faceAlloc() const { return faceCount() + (size_t)32 * 12 * GF; }
   size_t refCount(int rows) const { return (size_t)nEl * rows * B * cfg.n_runs; }
   cudaError_t ensureStage() {
     if (stage) return cudaSuccess;
@@ -511,13 +522,13 @@ struct edge_b200_ctx {
     return cudaSuccess;
   }
 
-  // the flux-solver pairs of the pre-mixed projections, as characteristic factors for the steps of
-  // a configuration whose kernels (GTS, or LTS for lts) mix through them (unless some face's pair is
-  // not of rank 3, found when the factors are built: the pairs themselves from then on until the
-  // element data changes), else as the pairs themselves
+  // the flux-solver pairs of the pre-mixed projections (weak form): as characteristic factors for the
+  // LTS steps of a configuration whose kernels mix through them (unless some face's pair is not of
+  // rank 3, found when the factors are built: the pairs themselves from then on until the element
+  // data changes), else as the pairs themselves
   cudaError_t ensureFsLR(bool lts = false) {
     if (!ks->premix()) return cudaSuccess;
-    const bool wantChar = (lts ? ks->charMixLts() : ks->charMix()) && !charRejected;
+    const bool wantChar = lts && ks->charMixLts() && !charRejected;
     if (!fsLRStale && fsLRChar == wantChar) return cudaSuccess;
     const int P = ks->fsPairStride();
     cudaError_t e = fsLR.fit(size_t(nEl) * 4 * 2 * P * realSize);
@@ -559,16 +570,65 @@ struct edge_b200_ctx {
     return cudaSuccess;
   }
 
+  // the coefficients of the strong-form step, for configurations that have it
+  cudaError_t ensureStep() {
+    if (!ks->strongSupported() || !stepStale || stepRejected) return cudaSuccess;
+    if (nEl >= (int64_t(1) << 28)) {  // beyond the packed gather table
+      stepRejected = true;
+      return cudaSuccess;
+    }
+    cudaError_t e;
+    const int E = ks->elementsPerCta();  // the layout's interleaving: whole groups of E elements
+    if ((e = fac.fit(size_t((nEl + E - 1) / E * E) * kFacLen * realSize)) || (e = gath.fit(size_t(nEl) * 4 * sizeof(uint32_t))) ||
+        (e = stepBad.fit(sizeof(int))))
+      return e;
+    // the count of faces not of rank 3 is read back once (no allocation of its own or device-wide
+    // synchronisation on the way: pools of a server set themselves up while others run)
+    int *bad = stepBad.as<int>(), nBad = 0;
+    if ((e = cudaMemsetAsync(bad, 0, sizeof(int), stream))) return e;
+    const int64_t work = (nEl * 4 + 31) / 32;  // 64 threads each
+    const int grid = (int)std::min<int64_t>(work, 148 * 64);
+    if (cfg.precision == 64)
+      kBuildStep<double><<<grid, 64, 0, stream>>>(fsE, starE, elFaEl, fId, vId, faType, nEl, cfg.order, E,
+                                                  fac.as<double>(), gath.as<uint32_t>(), bad);
+    else
+      kBuildStep<float><<<grid, 64, 0, stream>>>(fsE, starE, elFaEl, fId, vId, faType, nEl, cfg.order, E,
+                                                 fac.as<float>(), gath.as<uint32_t>(), bad);
+    if ((e = cudaGetLastError())) return e;
+    if ((e = cudaMemcpyAsync(&nBad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream))) return e;
+    if ((e = cudaStreamSynchronize(stream))) return e;
+    stepStale = false;
+    stepRejected = nBad != 0;
+    return cudaSuccess;
+  }
+  // what a GTS step of this context needs built
+  cudaError_t ensureGts() {
+    cudaError_t e = ensureStep();
+    return e || strong() ? e : ensureFsLR();
+  }
+  void dataChanged() {
+    fsLRStale = stepStale = true;
+    charRejected = stepRejected = false;
+  }
+
   int fail(cudaError_t e, const char *what) {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return EDGE_B200_EDEVICE;
   }
-  StepArgsRaw args(double dt) const {
+  // weak: for the weak-form kernels (LTS), whatever form the GTS steps take
+  StepArgsRaw args(double dt, bool weak = false) const {
     StepArgsRaw a;
     a.dofsE = dofsE;
     a.dofsA = dofsA;
     a.tDofs = keepTDofs ? tDofs : nullptr;
-    a.face = faceBuf(faceCur);
+    if (strong() && !weak) {
+      a.fac = fac.p;
+      a.gath = gath.as<uint32_t>();
+      a.face = outBuf(outCur);
+      a.wOwn = faceThird(2);
+    } else {
+      a.face = face;
+    }
     a.starE = starE;
     a.starA = starA;
     a.srcA = srcA;
@@ -662,13 +722,13 @@ int edge_b200_create(const edge_b200_cfg *cfg, int64_t n_el, edge_b200_ctx **out
   size_t rs = ctx->realSize;
   if ((e = cudaMalloc(&ctx->dofsE, ctx->dofsCount() * rs)) ||
       (cfg->n_rms && (e = cudaMalloc(&ctx->dofsA, ctx->dofsACount() * rs))) ||
-      (e = cudaMalloc(&ctx->face, ctx->faceCount() * rs))) {
+      (e = cudaMalloc(&ctx->face, ctx->faceAlloc() * rs))) {
     delete ctx;
     return e == cudaErrorMemoryAllocation ? EDGE_B200_ENOMEM : EDGE_B200_EDEVICE;
   }
   cudaMemsetAsync(ctx->dofsE, 0, ctx->dofsCount() * rs, ctx->stream);
   if (cfg->n_rms) cudaMemsetAsync(ctx->dofsA, 0, ctx->dofsACount() * rs, ctx->stream);
-  cudaMemsetAsync(ctx->face, 0, ctx->faceCount() * rs, ctx->stream);
+  cudaMemsetAsync(ctx->face, 0, ctx->faceAlloc() * rs, ctx->stream);
   *out = ctx;
   return EDGE_B200_OK;
 }
@@ -701,8 +761,7 @@ int edge_b200_upload_mesh(edge_b200_ctx *ctx, const int32_t *el_fa_el, const uin
   ctx->hFId.assign(fid_el_fa_el, fid_el_fa_el + n);
   ctx->hFaType.assign(el_fa_type, el_fa_type + n);
   ctx->meshSet = true;
-  ctx->fsLRStale = true;
-  ctx->charRejected = false;
+  ctx->dataChanged();
   return EDGE_B200_OK;
 }
 
@@ -728,8 +787,7 @@ int edge_b200_upload_element_data(edge_b200_ctx *ctx, const double *star_e, cons
   }
   EDGE_CUDA(cudaStreamSynchronize(s), "upload element data");
   ctx->dataSet = true;
-  ctx->fsLRStale = true;
-  ctx->charRejected = false;
+  ctx->dataChanged();
   return EDGE_B200_OK;
 }
 
@@ -751,8 +809,7 @@ int edge_b200_share_element_data(edge_b200_ctx *dst, const edge_b200_ctx *src) {
   for (int m = 0; m < 3; m++) ctx->omega[m] = src->omega[m];
   ctx->sharedData = true;
   ctx->dataSet = true;
-  ctx->fsLRStale = true;
-  ctx->charRejected = false;
+  ctx->dataChanged();
   return EDGE_B200_OK;
 }
 
@@ -1027,18 +1084,11 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
   if (!ctx->meshSet || !ctx->dataSet) return EDGE_B200_EINVAL;
   ctx->lastLts = false;
   cudaStream_t s = ctx->stream;
-  EDGE_CUDA(ctx->ensureFsLR(), "flux-solver pairs");
-  // whole GTS steps of a pre-mixing configuration without halo parts fold each neighbour step
-  // into the next local step; the split phases run the neighbour step on its own
-  const bool fused = phases == 3 && ctx->fusedOn && ctx->ks->fusedSupported() && ctx->nOwned == ctx->nEl;
-  if (fused) {
-    if (!ctx->faceAlt.p) {
-      EDGE_CUDA(ctx->faceAlt.fit(ctx->faceCount() * ctx->realSize), "second face buffer");
-      EDGE_CUDA(cudaMemsetAsync(ctx->faceAlt.p, 0, ctx->faceCount() * ctx->realSize, s), "second face buffer");
-    }
-  } else {
-    EDGE_CUDA(ctx->flush(), "pending neighbour step");
-  }
+  EDGE_CUDA(ctx->ensureGts(), "step coefficients");
+  // whole strong-form steps without halo parts fold each step's surface integrals into the next
+  // step's kernel; the split phases run them on their own
+  const bool fused = phases == 3 && ctx->fusedOn && ctx->strong() && ctx->nOwned == ctx->nEl;
+  if (!fused) EDGE_CUDA(ctx->flush(), "pending neighbour step");
   // receiver samples of every step (Receivers::getRecvTimeRel, io/Receivers.cpp:235-248)
   std::vector<int> stepFirst(n_steps + 1, 0);
   std::vector<double> tau;
@@ -1084,9 +1134,9 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
   for (int st = 0; st < n_steps; st++) {
     const int ns = stepFirst[st + 1] - stepFirst[st];
     if (fused) {
-      // the previous step's projections (their neighbour step still pending) in, this step's out
-      a.faceIn = ctx->pending ? ctx->faceBuf(ctx->faceCur) : nullptr;
-      a.face = ctx->faceBuf(ctx->faceCur ^ 1);
+      // the previous step's characteristics (still pending) in, this step's out
+      a.faceIn = ctx->pending ? ctx->outBuf(ctx->outCur) : nullptr;
+      a.face = ctx->outBuf(ctx->outCur ^ 1);
     }
     if ((phases & 1) && ns > 0 && ctx->nRecvGrp > 0) {
       RecvArgs r;
@@ -1103,8 +1153,7 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
       ctx->launches++;
     }
     if (phases & 1) {
-      EDGE_CUDA(ctx->launch(0, [&] { return fused ? ctx->ks->localFused(a, s) : ctx->ks->local(a, s); }),
-                "local kernel");
+      EDGE_CUDA(ctx->launch(0, [&] { return ctx->ks->local(a, s); }), "local kernel");
       ctx->launches++;
       if (ctx->src.nGrp > 0 && ctx->rangeSrc) {
         SrcArgs sa = ctx->src;
@@ -1122,7 +1171,7 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
     }
     if ((phases & 1) && ctx->rangeSrc) ctx->srcStep++;
     if (fused) {
-      ctx->faceCur ^= 1;
+      ctx->outCur ^= 1;
       ctx->pending = true;
     } else if (phases & 2) {
       EDGE_CUDA(ctx->launch(1, [&] { return ctx->ks->neigh(a, s); }), "neighbour kernel");
@@ -1184,11 +1233,14 @@ int64_t edge_b200_face_block_bytes(const edge_b200_ctx *ctx) {
 static int packFaces(edge_b200_ctx *ctx, int n, const int32_t *slots, void *buf, bool pack) {
   if (!ctx || n < 0 || (n && (!slots || !buf))) return EDGE_B200_EINVAL;
   if (n == 0) return EDGE_B200_OK;
-  const int64_t blk16 = edge_b200_face_block_bytes(ctx) / 16;
+  if (ctx->meshSet && ctx->dataSet) EDGE_CUDA(ctx->ensureGts(), "step coefficients");
+  // strong form: the three characteristic rows of the slot, at the start of its block
+  const bool st = ctx->strong();
+  const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16, blk16 = st ? stride16 / 3 : stride16;
   const int64_t total = (int64_t)n * blk16;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
-  kFacePack<<<grid, 256, 0, ctx->stream>>>(static_cast<uint4 *>(ctx->faceBuf(ctx->faceCur)), static_cast<uint4 *>(buf), slots,
-                                             n, blk16, ctx->nEl * 4, pack);
+  kFacePack<<<grid, 256, 0, ctx->stream>>>(static_cast<uint4 *>(st ? ctx->outBuf(ctx->outCur) : ctx->face),
+                                           static_cast<uint4 *>(buf), slots, n, blk16, stride16, ctx->nEl * 4, pack);
   EDGE_CUDA(cudaGetLastError(), pack ? "pack faces" : "unpack faces");
   return EDGE_B200_OK;
 }
@@ -1330,7 +1382,7 @@ int edge_b200_step_lts(edge_b200_ctx *ctx, double t, double dt_fun, int n_cycles
   }
   ctx->launches = 0;
   for (const Work &w : work) {
-    StepArgsRaw a = ctx->args(w.dt);
+    StepArgsRaw a = ctx->args(w.dt, true);
     a.elFirst = ctx->tgFirst[w.g];
     a.elCount = ctx->tgFirst[w.g + 1] - ctx->tgFirst[w.g];
     a.faceSum = ctx->faceSum.p;
@@ -1515,7 +1567,7 @@ int64_t edge_b200_last_launches(const edge_b200_ctx *ctx) { return ctx ? ctx->la
 
 int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]) {
   if (!ctx || !info) return EDGE_B200_EINVAL;
-  info[5] = (ctx->fusedOn && ctx->ks->fusedSupported() && ctx->nOwned == ctx->nEl) ? 1 : 0;
+  info[5] = (ctx->fusedOn && ctx->ks->premix() && ctx->nOwned == ctx->nEl) ? 1 : 0;
   info[0] = ctx->ks->elementsPerCta();
   info[1] = ctx->ks->premix() ? ((ctx->ks->charMix() && !ctx->charRejected) ? 2 : 1) : 0;
   info[2] = ctx->ks->fsPairStride();
@@ -1586,12 +1638,13 @@ struct edge_b200_batch {
     dfree(steps);
     dfree(activeDev);
   }
-  // contexts whose GTS steps fold each neighbour step into the next local step (as edge_b200_step
-  // does): within a call their steps alternate between the two face buffers
-  static bool fused(const edge_b200_ctx *c) { return c->fusedOn && c->ks->fusedSupported(); }
+  // contexts whose GTS steps fold each step's surface integrals into the next step's kernel (as
+  // edge_b200_step does): within a call their steps alternate between the two buffers of
+  // characteristics
+  static bool fused(const edge_b200_ctx *c) { return c->fusedOn && c->strong(); }
   // one GTS step of context k on its stream, its sources at t0 + tOff + steps[k] * dt. kind 0: a
-  // call's first step (fused contexts: nothing pending, projections out to faceAlt); 1: fused,
-  // pending projections in faceAlt, out to face; 2: in face, out to faceAlt. Other contexts take
+  // call's first step (fused contexts: nothing pending, characteristics out to buffer 1); 1: fused,
+  // pending ones in buffer 1, out to buffer 0; 2: in buffer 0, out to buffer 1. Other contexts take
   // a whole separate-kernel step (local, sources, neighbour) in each kind.
   cudaError_t issueStep(size_t k, int kind, double tOff) {
     edge_b200_ctx *ctx = ctxs[k];
@@ -1599,13 +1652,10 @@ struct edge_b200_batch {
     StepArgsRaw a = ctx->args(dt[k]);
     cudaError_t c;
     if (fu[k]) {
-      a.faceIn = kind == 0 ? nullptr : ctx->faceBuf(kind == 1 ? 1 : 0);
-      a.face = ctx->faceBuf(kind == 1 ? 0 : 1);
-      c = ctx->ks->localFused(a, s);
-    } else {
-      c = ctx->ks->local(a, s);
+      a.faceIn = kind == 0 ? nullptr : ctx->outBuf(kind == 1 ? 1 : 0);
+      a.face = ctx->outBuf(kind == 1 ? 0 : 1);
     }
-    if (c) return c;
+    if ((c = ctx->ks->local(a, s))) return c;
     if (ctx->src.nGrp > 0) {
       SrcArgs sa = ctx->src;
       sa.t = t0[k] + tOff;
@@ -1649,10 +1699,9 @@ struct edge_b200_batch {
                              origin)))
       return e;
     if ((e = cudaStreamSynchronize(origin))) return e;
-    // each context's step form for this graph and the direct launches around it (a context switched
-    // to fused steps after the batch was created, without its second face buffer, stays separate)
+    // each context's step form for this graph and the direct launches around it
     fu.assign(ctxs.size(), 0);
-    for (size_t k = 0; k < ctxs.size(); k++) fu[k] = fused(ctxs[k]) && ctxs[k]->faceAlt.p != nullptr;
+    for (size_t k = 0; k < ctxs.size(); k++) fu[k] = fused(ctxs[k]);
     if ((e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal))) return e;
     cudaError_t c = forkJoin([&](size_t k) {
       cudaError_t r = issueStep(k, 1, 0.0);
@@ -1677,9 +1726,16 @@ struct edge_b200_batch {
   // that nothing is pending when the call returns
   cudaError_t run(int n) {
     cudaError_t c;
+    // element data set since: coefficients again, and the graph with them
+    for (size_t k = 0; k < ctxs.size(); k++) {
+      edge_b200_ctx *ctx = ctxs[k];
+      if (!active[k] || !ctx->stepStale || !ctx->ks->strongSupported()) continue;
+      if ((c = ctx->ensureGts()) || (c = cudaStreamSynchronize(ctx->stream))) return c;
+      dirty = true;
+    }
     if (dirty && (c = capture())) return c;
     for (size_t k = 0; k < ctxs.size(); k++)
-      if (active[k] && fu[k]) ctxs[k]->faceCur = 0;  // nothing pending: only a relabelling
+      if (active[k] && fu[k]) ctxs[k]->outCur = 0;  // nothing pending: only a relabelling
     if ((c = forkJoin([&](size_t k) { return issueStep(k, 0, 0.0); }))) return c;
     if ((c = advance(1))) return c;
     for (int i = 0; i < (n - 1) / 2; i++)
@@ -1689,18 +1745,18 @@ struct edge_b200_batch {
       if ((c = forkJoin([&](size_t k) { return issueStep(k, 1, 0.0); }))) return c;
       if ((c = advance(1))) return c;
     }
-    // last written: faceAlt after kinds 0 and 2, face after kind 1
+    // last written: buffer 1 after kinds 0 and 2, buffer 0 after kind 1
     const int last = odd ? 0 : 1;
     c = forkJoin([&](size_t k) {
       edge_b200_ctx *ctx = ctxs[k];
       if (!fu[k]) return cudaSuccess;
       StepArgsRaw a = ctx->args(dt[k]);
-      a.face = ctx->faceBuf(last);
+      a.face = ctx->outBuf(last);
       return ctx->ks->neigh(a, streams[k]);
     });
     if (c) return c;
     for (size_t k = 0; k < ctxs.size(); k++)
-      if (active[k] && fu[k]) ctxs[k]->faceCur = last;
+      if (active[k] && fu[k]) ctxs[k]->outCur = last;
     return cudaSuccess;
   }
 };
@@ -1746,11 +1802,7 @@ int edge_b200_batch_create(edge_b200_ctx *const *ctxs, int n, const double *t0, 
   for (int k = 0; k < n && !e; k++) {
     edge_b200_ctx *c = ctxs[k];
     e = c->flush();
-    if (!e) e = c->ensureFsLR();
-    if (!e && edge_b200_batch::fused(c) && !c->faceAlt.p) {
-      e = c->faceAlt.fit(c->faceCount() * c->realSize);
-      if (!e) e = cudaMemsetAsync(c->faceAlt.p, 0, c->faceCount() * c->realSize, c->stream);
-    }
+    if (!e) e = c->ensureGts();
     if (!e) e = cudaEventRecord(b->joins[k], c->stream);
     if (!e) e = cudaStreamWaitEvent(b->origin, b->joins[k], 0);
   }
@@ -1801,7 +1853,7 @@ int edge_b200_autotune(edge_b200_ctx *ctx, double dt, int32_t caps[2]) {
   if (!ctx->meshSet || !ctx->dataSet || ctx->timing) return EDGE_B200_EINVAL;
   cudaStream_t s = ctx->stream;
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
-  EDGE_CUDA(ctx->ensureFsLR(), "flux-solver pairs");
+  EDGE_CUDA(ctx->ensureGts(), "step coefficients");
   const size_t rs = ctx->realSize;
   const size_t bytesE = ctx->dofsCount() * rs, bytesA = ctx->dofsACount() * rs;
   DevBuf save;

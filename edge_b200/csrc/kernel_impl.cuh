@@ -1,7 +1,7 @@
 // KernelSet implementation for one configuration; included by the inst_*.cu translation units.
 #pragma once
 #include "kernel_set.h"
-#include "kernels.cuh"
+#include "step.cuh"
 
 namespace edge_b200 {
 
@@ -9,7 +9,7 @@ template <typename T, int O, int R, int RM>
 class KernelSetImpl final : public KernelSet {
   using G = Geo<T, O, R, RM>;
   int numSms_ = 0, occLocal_ = 1, occNeigh_ = 1, occRecv_ = 1, occLocalLts_ = 1, occLocalSum_ = 1,
-      capLocal_ = 0, capNeigh_ = 0;
+      occStep_ = 1, occLift_ = 1, capLocal_ = 0, capNeigh_ = 0;
 
   static StepArgs<T> cast(const StepArgsRaw &a) {
     StepArgs<T> b;
@@ -41,6 +41,9 @@ class KernelSetImpl final : public KernelSet {
     b.firstTs = a.firstTs;
     b.fsLR = static_cast<const T *>(a.fsLR);
     b.fsChar = a.fsChar;
+    b.fac = static_cast<const T *>(a.fac);
+    b.gath = a.gath;
+    b.wOwn = static_cast<T *>(a.wOwn);
     b.faceIn = static_cast<const T *>(a.faceIn);
     b.grpDt = a.grpDt;
     return b;
@@ -61,18 +64,16 @@ class KernelSetImpl final : public KernelSet {
       return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLocal_, kLocal<T, O, R, RM, 0>, G::NT, smemLocal())))
       return e;
-    if constexpr (G::premix) {
-      if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smemLocal())))
+    if constexpr (RM == 0) {
+      using S = SGeo<T, O, R>;
+      if ((e = cudaFuncSetAttribute(kStep<T, O, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem)))
         return e;
-    }
-    if constexpr (G::charMix) {
-      if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 0, false, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemLocal())))
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occStep_, kStep<T, O, R>, S::NT, S::smem))) return e;
+      if ((e = cudaFuncSetAttribute(kLift<T, O, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smemLift)))
         return e;
-      if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 0, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smemLocal())))
-        return e;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLift_, kLift<T, O, R>, S::NT, S::smemLift))) return e;
+      occStep_ = occStep_ < 1 ? 1 : occStep_;
+      occLift_ = occLift_ < 1 ? 1 : occLift_;
     }
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occNeigh_, kNeigh<T, O, R, RM, G::premix>, G::NT, smemNeigh())))
       return e;
@@ -97,10 +98,10 @@ class KernelSetImpl final : public KernelSet {
         return e;
       occLocalSum_ = occLocalSum_ < 1 ? 1 : occLocalSum_;
       if constexpr (G::charMixLts) {
-        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 2, false, true>,
+        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 2, true>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smemLocalLts)))
           return e;
-        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 1, false, true>,
+        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 1, true>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smemLocalSums)))
           return e;
       }
@@ -124,37 +125,23 @@ class KernelSetImpl final : public KernelSet {
 
   cudaError_t local(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
-    if constexpr (G::charMix) {
-      if (a.fsChar) {
-        kLocal<T, O, R, RM, 0, false, true><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
+    if constexpr (RM == 0) {
+      using S = SGeo<T, O, R>;
+      if (a.fac) {
+        kStep<T, O, R><<<grid(a.elCount, capLocal_ > 0 ? capLocal_ : numSms_ * occStep_), S::NT, S::smem, s>>>(cast(a));
         return cudaGetLastError();
       }
     }
     kLocal<T, O, R, RM, 0><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
     return cudaGetLastError();
   }
-  cudaError_t localFused(const StepArgsRaw &a, cudaStream_t s) override {
-    if constexpr (G::premix) {
-      if (a.elCount < 1) return cudaSuccess;
-      if constexpr (G::charMix) {
-        if (a.fsChar) {
-          kLocal<T, O, R, RM, 0, true, true><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
-          return cudaGetLastError();
-        }
-      }
-      kLocal<T, O, R, RM, 0, true><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
-  }
-  bool fusedSupported() const override { return G::premix; }
+  bool strongSupported() const override { return RM == 0; }
   cudaError_t localLts(const StepArgsRaw &a, cudaStream_t s) override {
     if constexpr (G::ltsOk) {
       if (a.elCount < 1) return cudaSuccess;
       if constexpr (G::charMixLts) {
         if (a.fsChar) {
-          kLocal<T, O, R, RM, 2, false, true>
+          kLocal<T, O, R, RM, 2, true>
               <<<grid(a.elCount, numSms_ * occLocalLts_), G::NT, G::smemLocalLts, s>>>(cast(a));
           return cudaGetLastError();
         }
@@ -170,7 +157,7 @@ class KernelSetImpl final : public KernelSet {
       if (a.elCount < 1) return cudaSuccess;
       if constexpr (G::charMixLts) {
         if (a.fsChar) {
-          kLocal<T, O, R, RM, 1, false, true>
+          kLocal<T, O, R, RM, 1, true>
               <<<grid(a.elCount, numSms_ * occLocalSum_), G::NT, G::smemLocalSums, s>>>(cast(a));
           return cudaGetLastError();
         }
@@ -188,6 +175,13 @@ class KernelSetImpl final : public KernelSet {
   bool charMixLts() const override { return G::charMixLts; }
   cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
+    if constexpr (RM == 0) {
+      using S = SGeo<T, O, R>;
+      if (a.fac) {
+        kLift<T, O, R><<<grid(a.elCount, capNeigh_ > 0 ? capNeigh_ : numSms_ * occLift_), S::NT, S::smemLift, s>>>(cast(a));
+        return cudaGetLastError();
+      }
+    }
     kNeigh<T, O, R, RM, G::premix><<<grid(a.elCount, ctasNeigh()), G::NT, smemNeigh(), s>>>(cast(a));
     return cudaGetLastError();
   }

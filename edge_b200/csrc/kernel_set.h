@@ -26,10 +26,14 @@ struct StepArgsRaw {
   int firstTs = 0;
   // per element face fsE[0] and the face reader's fsE[1] in the configuration's precision, each
   // padded to 16 bytes: [nEl][4][2][fsPairStride()] (premix); fsChar: their characteristic
-  // factors instead (charMix)
+  // factors instead (charMixLts)
   const void *fsLR = nullptr;
   int fsChar = 0;
-  // fused GTS steps: the previous step's face projections whose neighbour step is still pending
+  // strong-form GTS steps (StepArgs): coefficients (null: the weak-form kernels), gather table, own
+  // characteristics, and the characteristics of the previous step that are still pending
+  const void *fac = nullptr;
+  const uint32_t *gath = nullptr;
+  void *wOwn = nullptr;
   const void *faceIn = nullptr;
   // per element group time steps of the GTS local step (merged simulations), or null
   const double *grpDt = nullptr;
@@ -39,10 +43,12 @@ class KernelSet {
  public:
   virtual ~KernelSet() {}
   virtual cudaError_t init(int device) = 0;  // sets smem attributes, sizes the persistent grids
+  // GTS local step: in strong form when a.fac is given (the pending surface integrals of a.faceIn
+  // first), else in weak form
   virtual cudaError_t local(const StepArgsRaw &a, cudaStream_t s) = 0;
-  // the local step with the pending neighbour step of the previous one folded in (a.faceIn)
-  virtual cudaError_t localFused(const StepArgsRaw &a, cudaStream_t s) = 0;
-  virtual bool fusedSupported() const = 0;
+  // the configuration has the strong-form step (step.cuh), whose closing half neigh runs when a.fac
+  // is given
+  virtual bool strongSupported() const = 0;
   // local step with the LTS face buffers (the half-step time integral needs one more tile)
   virtual cudaError_t localLts(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the same without half-step integrals, for elements without a smaller neighbour (no extra tile)
@@ -51,10 +57,10 @@ class KernelSet {
   // GTS face projections leave the local kernel mixed with the reader's flux solver (fsLR)
   virtual bool premix() const = 0;
   virtual int fsPairStride() const = 0;
-  // the GTS local kernel mixes face projections through the rank-3 factors of the flux-solver
-  // pairs when fsLR holds them (StepArgsRaw::fsChar)
+  // room for the characteristic rows beside the pre-mixing buffers
   virtual bool charMix() const = 0;
-  // the LTS local kernels do the same (both of their tiles of characteristic rows fit)
+  // the LTS local kernels mix face projections through the rank-3 factors of the flux-solver pairs
+  // when fsLR holds them (StepArgsRaw::fsChar; both of their tiles of characteristic rows fit)
   virtual bool charMixLts() const = 0;
   virtual cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the neighbour step over the buffers the LTS local kernels wrote (pre-mixed where those

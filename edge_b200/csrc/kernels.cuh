@@ -55,12 +55,17 @@ struct StepArgs {
   // its face reader applies (fsE[1] of the face neighbour at its face, or the element's own for a
   // free surface; zeros for outflow) in T, each padded to 16 bytes (Geo::FSP): [nEl][4][2][FSP];
   // null: gathered through the connectivity. fsChar: fsLR holds the characteristic factors of
-  // those pairs instead (Geo::charMix: V [9][4], then per quantity {U0[q][0..2], U1[q][0..2], 0, 0})
+  // those pairs instead (LTS, Geo::charMixLts: V [9][4], then per quantity {U0[q][0..2], U1[q][0..2], 0, 0})
   const T *fsLR;
   int fsChar;
-  // fused GTS steps (kLocal<..., FUSED>, kRecv): the previous step's pre-mixed face projections,
-  // whose neighbour fluxes are added to the DOF rows before the recursion (the previous step's
-  // neighbour step runs here), or null when none are pending
+  // strong-form GTS steps (step.cuh): the coefficients of the elements, null for the
+  // kernels of this file; per face the packed (neighbour * 4 + its face) * 4 + orientation or
+  // 0xffffffff; the elements' own characteristics; face then holds those they
+  // write for their neighbours, and faceIn the previous step's, still to be added to the DOF rows,
+  // or null when none are pending
+  const T *fac;
+  const uint32_t *gath;
+  T *wOwn;
   const T *faceIn;
   // GTS local step with a time step per element group (g = 0 .. of the launch range: E elements
   // each) instead of dt, or null: several simulations merged into one context step together
@@ -249,8 +254,13 @@ __device__ __forceinline__ void copyRows(T *tile, const T *base, int64_t e, int 
 #pragma unroll
   for (int it = 0; it < CPRB; it++) {
     const int k = it * R + r;
-    const int row = k / CPRB, col = k % CPRB;
-    cpAsync16(dst + row * S + col * W, blk + row * GB + col * W);
+    if constexpr (S == GB) {
+      // rows without padding: one offset for the whole block (no row and column to keep per chunk)
+      cpAsync16(dst + k * W, blk + k * W);
+    } else {
+      const int row = k / CPRB, col = k % CPRB;
+      cpAsync16(dst + row * S + col * W, blk + row * GB + col * W);
+    }
   }
 }
 
@@ -273,14 +283,11 @@ __device__ __forceinline__ void storeRowsCoalesced(const T *tile, T *blk, int q,
   for (int it = 0; it < CPR; it++) {
     const int k = it * R + r;
     const int row = k / CPR, col = k % CPR;
-    T v[4];
-    if constexpr (sizeof(T) == 4) {
-      ld4<T>(src + row * S + col * W, v);
-      *reinterpret_cast<float4 *>(blk + row * G + col * W) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-      const double2 d = *reinterpret_cast<const double2 *>(src + row * S + col * W);
-      *reinterpret_cast<double2 *>(blk + row * G + col * W) = d;
-    }
+    const int from = S == G ? k * W : row * S + col * W;
+    if constexpr (sizeof(T) == 4)
+      *reinterpret_cast<float4 *>(blk + k * W) = *reinterpret_cast<const float4 *>(src + from);
+    else
+      *reinterpret_cast<double2 *>(blk + k * W) = *reinterpret_cast<const double2 *>(src + from);
   }
 }
 
@@ -1053,46 +1060,6 @@ __device__ __forceinline__ int neighOri(const FaceMeta &m) {
 }
 
 
-// the neighbour flux of face FA through pre-mixed projections read straight from global memory
-// (this warp's quantity row, this lane's run): the arithmetic of the neighbour kernel's
-// neighApplyMixed, for kernels that fold a pending neighbour step into their DOF rows
-template <typename T, int O, int R, int RM, int FA>
-__device__ __forceinline__ void neighFluxFace(const T *faceIn, const FaceMeta &m, int64_t e, int q, int r,
-                                              bool valid, T *acc) {
-  using G = Geo<T, O, R, RM>;
-  constexpr int F = G::F;
-  const int ty = m.type(FA);
-  if (!valid || ty == FT_OUTFLOW || q >= 9) return;
-  const int64_t src = ty == FT_INNER ? int64_t(m.src[FA]) : e * 4 + FA;
-  T x[F];
-  ldRowG<T, F>(gRow<T, R, G::GF>(faceIn, src, 9, q, r), x, true);
-  if (ty == FT_INNER) {
-    T o[F];
-#pragma unroll
-    for (int j = 0; j < F; j++) o[j] = T(0);
-    const int v = neighOri<O, FA>(m);
-    if (v == 0)
-      OriMul<O, 0>::template run<T>(x, o);
-    else if (v == 1)
-      OriMul<O, 1>::template run<T>(x, o);
-    else
-      OriMul<O, 2>::template run<T>(x, o);
-    FluxTMul<O, FA>::template run<T>(o, acc);
-  } else {
-    FluxTMul<O, FA>::template run<T>(x, acc);
-  }
-}
-template <typename T, int O, int R, int RM>
-__device__ __forceinline__ void neighFluxDirect(const StepArgs<T> &a, const T *faceIn, int64_t e, int q, int r,
-                                                bool valid, T *acc) {
-  FaceMeta m;
-  m.load(a, e, valid);
-  neighFluxFace<T, O, R, RM, 0>(faceIn, m, e, q, r, valid, acc);
-  neighFluxFace<T, O, R, RM, 1>(faceIn, m, e, q, r, valid, acc);
-  neighFluxFace<T, O, R, RM, 2>(faceIn, m, e, q, r, valid, acc);
-  neighFluxFace<T, O, R, RM, 3>(faceIn, m, e, q, r, valid, acc);
-}
-
 // ------------------------------------------------------------------------------------------------
 // local step: CK, volume, local surface, face projections (AderDg::local, AderDg.hpp:338-534)
 // ------------------------------------------------------------------------------------------------
@@ -1356,9 +1323,8 @@ __device__ __forceinline__ void facesSplit(const StepArgs<T> &a, const T *TI, T 
 
 // LTS as in localFace; mode 2 keeps the half-step integral in one more tile (one CTA per SM), mode
 // 1 runs on the elements of a time group without a smaller neighbour
-// FUSED (GTS, pre-mixing configurations): the previous step's neighbour fluxes (a.faceIn, when
-// pending) are added to each group's DOF rows first, and the completed rows stored back
-template <typename T, int O, int R, int RM, int LTS, bool FUSED = false, bool CHAR = false>
+// CHAR (LTS): the mixes go through the characteristic factors
+template <typename T, int O, int R, int RM, int LTS, bool CHAR = false>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O, R, RM>::minCtasLocal)
     kLocal(StepArgs<T> a) {
   using G = Geo<T, O, R, RM>;
@@ -1444,20 +1410,6 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         else
 #pragma unroll
           for (int n = 0; n < B; n++) v[n] = T(0);
-        if constexpr (FUSED) {
-          if (a.faceIn) {
-            neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
-            // the completed rows back to the DOFs (the volume integral reads them again)
-            T *p = rowPtr<T, SB>(X, q, l);
-            stRow<T, B>(p, v);
-#pragma unroll
-            for (int n = B; n < G::GB; n++) p[n] = T(0);
-            __syncwarp();
-            if (valid)
-              storeRowsCoalesced<T, R, G::GB, SB>(X, a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q, eo, r);
-            __syncwarp();
-          }
-        }
         stRow<T, B>(rowPtr<T, SB>(X, q, l), v);
       } else {
         ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, ev, 9, q, r), v, valid);
@@ -2057,6 +2009,20 @@ __device__ __forceinline__ void recvAll(T *X, T *TI, T *XA, T *TIA, int q, int l
   }
 }
 
+// (step.cuh)
+constexpr int kFacLen = 540;
+template <typename T, int O, int R>
+struct SGeo;
+template <typename T, int O, int R>
+__device__ __forceinline__ void liftRow(const StepArgs<T> &a, const T *in, T *wt, int t, int l, int64_t e, int r,
+                                        bool valid);
+template <typename T, int O, int R>
+__device__ __forceinline__ const T *facPtr(const T *fac, int64_t e);
+template <typename T, int O, int R>
+struct FacU;
+template <typename T, int O, int R, typename Z>
+__device__ __forceinline__ void liftApply(const T *wt, const Z &U, int l, T *acc);
+
 template <typename T, int O, int R, int RM>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, RecvArgs rv) {
   using G = Geo<T, O, R, RM>;
@@ -2081,9 +2047,17 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
   if (q < 9) {
     T v[B];
     ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, ev, 9, q, r), v, valid);
-    // a pending neighbour step (fused GTS steps) completes the rows first
+    // pending characteristics of a strong-form step complete the rows first (their tile lies over
+    // X and TI, which are written only after every warp has read it)
     if constexpr (RM == 0)
-      if (a.faceIn) neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
+      if (a.faceIn) {
+        static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
+        liftRow<T, O, R>(a, a.faceIn, X, q, l, ev, r, valid);
+        if (q < 3) liftRow<T, O, R>(a, a.faceIn, X, q + 9, l, ev, r, valid);
+        __syncthreads();
+        liftApply<T, O, R>(X, FacU<T, O, R>{facPtr<T, O, R>(a.fac, ev), q}, l, v);
+        __syncthreads();
+      }
     stRow<T, B>(rowPtr<T, SB>(X, q, l), v);
     if constexpr (G::tiSmem)
       stRow<T, B>(rowPtr<T, SB>(TI, q, l), zero);

@@ -17,6 +17,8 @@ it from shared memory with 128-bit loads (e.g. a star-matrix mix whose loads ser
 directions), and groups of rows without non-zeros are skipped entirely. The other two take
 register arrays:
 * ``FluxTMul<O,FA>``  acc[n] += sum_j s[j] * fluxT'_FA[j][n]         (lift from face FA)
+* ``FluxLC``, ``FluxTC``, ``FluxPairC``  the face products in chunks of four face modes, faces 2 and 3
+  together (chunk_structs, below)
 * ``OriMul<O,V>``     s[j]   += sum_k x[k] * (Mface^-1 Ori_V)[k][j]  (V: reflection of the face)
 
 Face bases. Each local face FA of every element keeps its projections in the hierarchical triangle
@@ -29,6 +31,13 @@ reference's vertex-id map (a reflection, tools/edge_pre/types/Tet.py faToFa); wi
 the sigma_FA that is again one of the three reflections, V = ``kFacePerm[O-2][fo][FA][v]``. The
 flux operators are the reference's up to this change of face basis, which the lifted flux does
 not see.
+
+Mirrored faces. Swapping the first two vertices of the reference tet maps face 2 to face 3 and
+multiplies basis function phi_(p1,p2,p3) by (-1)^p1, so with the rotations chosen above
+fluxL'_3[k][j] = S[j] (-1)^p1(k) fluxL'_2[k][j] with signs S[j]: the products of even and odd k with
+face 2's matrix, a and b, give both projections (a + b and S (a - b)), and the lift of both faces
+is one product with face 2's fluxT' of s2 + S s3 (even n) or s2 - S s3 (odd n). At order 5 the four
+faces then take 474 instead of 748 products each way (checked exactly when the code is generated).
 
 Derivative directions. The stiffness products run in the reference-coordinate derivative directions
 a = 0, 1, 2 given by the rows of ``DIRS`` (K'_a = sum_dim DIRS[a][dim] K_dim) instead of xi1, xi2,
@@ -151,6 +160,88 @@ def struct_fused(name, params, body, acc="acc"):
     return s
 
 
+def mode_parity(order):
+    """(-1)^p1 of every tet mode (the sign under the swap of the first two vertices)."""
+    return [-1 if p1 % 2 else 1 for d in range(order) for p1 in range(d + 1) for _ in range(d - p1 + 1)]
+
+
+def pair_signs(order, l2, l3):
+    """S[j] with l3[k][j] = S[j] (-1)^p1(k) l2[k][j] for every k (both fluxL' [B][F]), or None."""
+    par = mode_parity(order)
+    out = []
+    for j in range(len(l2[0])):
+        sj = [s for s in (1, -1) if all(l3[k][j] == s * par[k] * l2[k][j] for k in range(len(l2)))]
+        if not sj:
+            return None
+        out.append(sj[0])
+    return out
+
+
+def sum_rows(dst, rows, x, neg=False):
+    """``dst = sum of x[k] * entry`` over (k, entry), as one multiplication and FMAs; [] without rows."""
+    out = []
+    for i, (k, v) in enumerate(rows):
+        out.append(f"      {dst} = {x}[{k}] * {lit(v)};" if i == 0 else f"      {dst} = fmaT({x}[{k}], {lit(v)}, {dst});")
+    return out
+
+
+def project_chunk(order, mat, js, keep, dst):
+    """dst[i] = sum over the modes k that `keep` admits of TI_k mat[k][js[i]], where TI_k is ti[k]
+    below B(O-1) and dt q[k] from there on (no time derivative reaches those modes)."""
+    nk, nb, lines = dgmat.n_modes_tet(order - 1), len(mat), []
+    for i, j in enumerate(js):
+        hi = [(k, mat[k][j]) for k in range(nk, nb) if keep(k) and mat[k][j] != 0]
+        lo = [(k, mat[k][j]) for k in range(nk) if keep(k) and mat[k][j] != 0]
+        lines += sum_rows(f"{dst}[{i}]", hi, "q")
+        if hi:
+            lines.append(f"      {dst}[{i}] *= dt;")
+            lines += [f"      {dst}[{i}] = fmaT(ti[{k}], {lit(v)}, {dst}[{i}]);" for k, v in lo]
+        else:
+            lines += sum_rows(f"{dst}[{i}]", lo, "ti") or [f"      {dst}[{i}] = T(0);"]
+    lines += [f"      {dst}[{i}] = T(0);" for i in range(len(js), 4)]
+    return lines
+
+
+def chunk_structs(order, fb):
+    """The face products in chunks of four face modes, which keep few values in registers at a time:
+    ``FluxLC<O,FA,C>`` / ``FluxTC<O,FA,C>`` project on and lift from modes [4C, 4C + 4) of face 0 or 1,
+    ``FluxPairC<O,C>`` those of faces 2 and 3 together."""
+    par = mode_parity(order)
+    sg = pair_signs(order, fb[2][1], fb[3][1])
+    l2, t2, t3 = fb[2][1], fb[2][2], fb[3][2]
+    nb, nf = len(l2), len(sg)
+    assert all(t3[j][n] == sg[j] * par[n] * t2[j][n] for j in range(nf) for n in range(nb)), "lift is mirrored too"
+    sig_l = "  static __device__ __forceinline__ void run(const T *__restrict__ ti, const T *__restrict__ q, T dt, T *__restrict__ s) {"
+    s = []
+    for c in range((nf + 3) // 4):
+        js = list(range(4 * c, min(4 * c + 4, nf)))
+        for f in (0, 1):
+            s += [f"template <> struct FluxLC<{order}, {f}, {c}> {{", "  template <typename T>", sig_l]
+            s += project_chunk(order, fb[f][1], js, lambda k: True, "s") + ["  }", "};", ""]
+            s += [f"template <> struct FluxTC<{order}, {f}, {c}> {{", "  template <typename T>",
+                  "  static __device__ __forceinline__ void run(const T *__restrict__ s, T *__restrict__ acc) {"]
+            s += [f"    acc[{n}] = fmaT(s[{i}], {lit(fb[f][2][j][n])}, acc[{n}]);" for i, j in enumerate(js)
+                  for n in range(nb) if fb[f][2][j][n] != 0]
+            s += ["  }", "};", ""]
+        s += [f"template <> struct FluxPairC<{order}, {c}> {{",
+              "  // projections of faces 2 and 3: a + b and S (a - b), a of the even and b of the odd modes", "  template <typename T>",
+              "  static __device__ __forceinline__ void project(const T *__restrict__ ti, const T *__restrict__ q, T dt, T *__restrict__ p2, T *__restrict__ p3) {",
+              "      T a[4], b[4];"]
+        s += project_chunk(order, l2, js, lambda k: par[k] > 0, "a") + project_chunk(order, l2, js, lambda k: par[k] < 0, "b")
+        s += [f"      p2[{i}] = a[{i}] + b[{i}]; p3[{i}] = {f'a[{i}] - b[{i}]' if sg[j] > 0 else f'b[{i}] - a[{i}]'};"
+              for i, j in enumerate(js)]
+        s += [f"      p2[{i}] = p3[{i}] = T(0);" for i in range(len(js), 4)]
+        s += ["  }", "  // lift: s2 + S s3 into the even modes, s2 - S s3 into the odd ones", "  template <typename T>",
+              "  static __device__ __forceinline__ void lift(const T *__restrict__ s2, const T *__restrict__ s3, T *__restrict__ acc) {"]
+        for i, j in enumerate(js):
+            p, m = ("+", "-") if sg[j] > 0 else ("-", "+")
+            s.append(f"    {{ const T u = s2[{i}] {p} s3[{i}], v = s2[{i}] {m} s3[{i}];")
+            s += [f"      acc[{n}] = fmaT({'u' if par[n] > 0 else 'v'}, {lit(t2[j][n])}, acc[{n}]);" for n in range(nb) if t2[j][n] != 0]
+            s.append("    }")
+        s += ["  }", "};", ""]
+    return s
+
+
 def main(out=None):
     here = os.path.dirname(os.path.abspath(__file__))
     out = out or os.path.join(here, "csrc", "gen", "dg_sparse.cuh")
@@ -165,6 +256,9 @@ def main(out=None):
          "template <int O> struct VolMul;",
          "template <int O, int FA> struct FluxLMul;",
          "template <int O, int FA> struct FluxTMul;",
+         "template <int O, int FA, int C> struct FluxLC;",
+         "template <int O, int FA, int C> struct FluxTC;",
+         "template <int O, int C> struct FluxPairC;",
          "template <int O, int V> struct OriMul;", ""]
     nm = dgmat.n_modes_tet
     tables = []
@@ -183,6 +277,7 @@ def main(out=None):
         for f in range(4):
             s += struct_fused("FluxLMul", f"{o}, {f}", block_rows4([fb[f][1]], B, F, "s"), "s")
             s += struct("FluxTMul", f"{o}, {f}", block("", None, None, fb[f][2], F, B, "s", "acc"), "s", "acc")
+        s += chunk_structs(o, fb)
         # face orientation: Mface^-1 Ori_v of the three reflections
         ori = exact_orientations(o)
         for v in range(3):
@@ -258,7 +353,7 @@ def perm_matrix(order, i):
 
 def face_bases(order):
     """Per face FA: (sigma_FA, fluxL'_FA [B][F], fluxT'_FA [F][B]) with the sparsest face matrices
-    (ties: the lowest permutation index)."""
+    (ties: the lowest permutation index); face 3 takes the rotation that mirrors face 2's."""
     ex = dgmat.exact_matrices(order)
     nb, nf = dgmat.n_modes_tet(order), dgmat.n_modes_tri(order)
     out = []
@@ -269,6 +364,8 @@ def face_bases(order):
             q = perm_matrix(order, i)
             pp = [[sum(q[m][j] * proj[k][j] for j in range(nf) if q[m][j]) for m in range(nf)] for k in range(nb)]
             nnz = sum(1 for k in range(nb) for m in range(nf) if pp[k][m] != 0)
+            if f == 3 and pair_signs(order, out[2][1], pp) is None:
+                continue
             if best is None or nnz < best[0]:
                 best = (nnz, i, pp)
         _, i, pp = best
