@@ -578,21 +578,22 @@ struct edge_b200_ctx {
       return cudaSuccess;
     }
     cudaError_t e;
+    const int len = cfg.n_rms ? FacL<3>::src + 12 * cfg.n_rms + 288 : FacL<0>::len;
     const int E = ks->elementsPerCta();  // the layout's interleaving: whole groups of E elements
-    if ((e = fac.fit(size_t((nEl + E - 1) / E * E) * kFacLen * realSize)) || (e = gath.fit(size_t(nEl) * 4 * sizeof(uint32_t))) ||
+    if ((e = fac.fit(size_t((nEl + E - 1) / E * E) * len * realSize)) || (e = gath.fit(size_t(nEl) * 4 * sizeof(uint32_t))) ||
         (e = stepBad.fit(sizeof(int))))
       return e;
     // the count of faces not of rank 3 is read back once (no allocation of its own or device-wide
     // synchronisation on the way: pools of a server set themselves up while others run)
     int *bad = stepBad.as<int>(), nBad = 0;
     if ((e = cudaMemsetAsync(bad, 0, sizeof(int), stream))) return e;
-    const int64_t work = (nEl * 4 + 31) / 32;  // 64 threads each
-    const int grid = (int)std::min<int64_t>(work, 148 * 64);
+    const int64_t work = (nEl * 8 + kTeams * kBuildWarps - 1) / (kTeams * kBuildWarps);
+    const int grid = (int)std::min<int64_t>(work, 148 * 32);
     if (cfg.precision == 64)
-      kBuildStep<double><<<grid, 64, 0, stream>>>(fsE, starE, elFaEl, fId, vId, faType, nEl, cfg.order, E,
+      kBuildStep<double><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
                                                   fac.as<double>(), gath.as<uint32_t>(), bad);
     else
-      kBuildStep<float><<<grid, 64, 0, stream>>>(fsE, starE, elFaEl, fId, vId, faType, nEl, cfg.order, E,
+      kBuildStep<float><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
                                                  fac.as<float>(), gath.as<uint32_t>(), bad);
     if ((e = cudaGetLastError())) return e;
     if ((e = cudaMemcpyAsync(&nBad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream))) return e;
@@ -1574,6 +1575,12 @@ int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]) {
   info[3] = ctx->ks->ctasLocal();
   info[4] = ctx->ks->ctasNeigh();
   return EDGE_B200_OK;
+}
+
+int edge_b200_step_form(edge_b200_ctx *ctx) {
+  if (!ctx || !ctx->meshSet || !ctx->dataSet) return EDGE_B200_EINVAL;
+  EDGE_CUDA(ctx->ensureGts(), "step coefficients");
+  return ctx->strong() ? 1 : 0;
 }
 
 int edge_b200_set_timing(edge_b200_ctx *ctx, int enable) {

@@ -1,7 +1,7 @@
 // KernelSet implementation for one configuration; included by the inst_*.cu translation units.
 #pragma once
 #include "kernel_set.h"
-#include "step.cuh"
+#include "step_visc.cuh"
 
 namespace edge_b200 {
 
@@ -10,6 +10,14 @@ class KernelSetImpl final : public KernelSet {
   using G = Geo<T, O, R, RM>;
   int numSms_ = 0, occLocal_ = 1, occNeigh_ = 1, occRecv_ = 1, occLocalLts_ = 1, occLocalSum_ = 1,
       occStep_ = 1, occLift_ = 1, capLocal_ = 0, capNeigh_ = 0;
+
+  // attenuation: the strong-form step where the anelastic rows fit its shared memory
+  static constexpr bool viscStrong = [] {
+    if constexpr (RM == 3)
+      return VGeo<T, O, R, RM>::ok;
+    else
+      return false;
+  }();
 
   static StepArgs<T> cast(const StepArgsRaw &a) {
     StepArgs<T> b;
@@ -64,6 +72,19 @@ class KernelSetImpl final : public KernelSet {
       return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLocal_, kLocal<T, O, R, RM, 0>, G::NT, smemLocal())))
       return e;
+    if constexpr (viscStrong) {
+      using V = VGeo<T, O, R, RM>;
+      if ((e = cudaFuncSetAttribute(kStepVisc<T, O, R, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V::smem)))
+        return e;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occStep_, kStepVisc<T, O, R, RM>, V::NT, V::smem))) return e;
+      if ((e = cudaFuncSetAttribute(kLiftVisc<T, O, R, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)V::smemLift)))
+        return e;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLift_, kLiftVisc<T, O, R, RM>, V::NT, V::smemLift)))
+        return e;
+      occStep_ = occStep_ < 1 ? 1 : occStep_;
+      occLift_ = occLift_ < 1 ? 1 : occLift_;
+    }
     if constexpr (RM == 0) {
       using S = SGeo<T, O, R>;
       if ((e = cudaFuncSetAttribute(kStep<T, O, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem)))
@@ -125,6 +146,14 @@ class KernelSetImpl final : public KernelSet {
 
   cudaError_t local(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
+    if constexpr (viscStrong) {
+      using V = VGeo<T, O, R, RM>;
+      if (a.fac) {
+        kStepVisc<T, O, R, RM>
+            <<<grid(a.elCount, capLocal_ > 0 ? capLocal_ : numSms_ * occStep_), V::NT, V::smem, s>>>(cast(a));
+        return cudaGetLastError();
+      }
+    }
     if constexpr (RM == 0) {
       using S = SGeo<T, O, R>;
       if (a.fac) {
@@ -135,7 +164,7 @@ class KernelSetImpl final : public KernelSet {
     kLocal<T, O, R, RM, 0><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
     return cudaGetLastError();
   }
-  bool strongSupported() const override { return RM == 0; }
+  bool strongSupported() const override { return RM == 0 || viscStrong; }
   cudaError_t localLts(const StepArgsRaw &a, cudaStream_t s) override {
     if constexpr (G::ltsOk) {
       if (a.elCount < 1) return cudaSuccess;
@@ -175,6 +204,14 @@ class KernelSetImpl final : public KernelSet {
   bool charMixLts() const override { return G::charMixLts; }
   cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
+    if constexpr (viscStrong) {
+      using V = VGeo<T, O, R, RM>;
+      if (a.fac) {
+        kLiftVisc<T, O, R, RM>
+            <<<grid(a.elCount, capNeigh_ > 0 ? capNeigh_ : numSms_ * occLift_), V::NT, V::smemLift, s>>>(cast(a));
+        return cudaGetLastError();
+      }
+    }
     if constexpr (RM == 0) {
       using S = SGeo<T, O, R>;
       if (a.fac) {

@@ -1980,20 +1980,31 @@ struct RecvArgs {
   double *buf;             // [nRecv][maxBuf][9][R]
 };
 
+// Receivers of an element whose sums over the modes stay in registers until every derivative is there
+// (their samples are then written once; the others' are added to in device memory level by level)
+constexpr int kRecvHeld = 2;
+
 template <typename T, int O, int R, int RM, int D>
 __device__ __forceinline__ void recvAll(T *X, T *TI, T *XA, T *TIA, int q, int l, const ElemCoef<T, RM> &c,
                                         const double *omega, T dt, T sca, const RecvArgs &rv, int i0, int i1,
-                                        bool valid, int r, T *tIr, T (*tIAr)[nModes(O)]) {
+                                        bool valid, int r, T *tIr, T (*tIAr)[nModes(O)], double (*held)[O]) {
   constexpr int B = nModes(O), SB = Geo<T, O, R, RM>::SB;
   // value[i][j][q][r] += tau_j^D / D! * sum_{n < B(O-D)} basis_i[n] der_D[q][n]  (CK modes only,
   // even with anelasticity: TimePred.hpp:149)
   if (q < 9 && valid) {
     constexpr int NCK = nModes(O - D);
     const T *xr = rowPtr<T, SB>(X, q, l);
-    for (int i = i0; i < i1; i++) {
+    const auto sum = [&](int i) {
       double dotv = 0;
 #pragma unroll
-      for (int n = 0; n < NCK; n++) dotv += rv.basis[i * B + n] * double(xr[n]);
+      for (int n = 0; n < NCK; n++) dotv += __ldg(rv.basis + i * B + n) * double(xr[n]);
+      return dotv;
+    };
+#pragma unroll
+    for (int h = 0; h < kRecvHeld; h++)
+      if (i0 + h < i1) held[h][D] = sum(i0 + h);
+    for (int i = i0 + kRecvHeld; i < i1; i++) {
+      const double dotv = sum(i);
       for (int j = 0; j < rv.nSamples; j++) {
         double cf = 1.0;
         for (int k = 1; k <= D; k++) cf *= rv.tau[j] / k;
@@ -2005,20 +2016,32 @@ __device__ __forceinline__ void recvAll(T *X, T *TI, T *XA, T *TIA, int q, int l
   if constexpr (D + 1 < O) {
     sca = sca * dt / T(D + 2);
     CkStep<T, O, R, RM, D + 1>::run(X, TI, XA, TIA, q, l, c, omega, sca, tIr, tIAr);
-    recvAll<T, O, R, RM, D + 1>(X, TI, XA, TIA, q, l, c, omega, dt, sca, rv, i0, i1, valid, r, tIr, tIAr);
+    recvAll<T, O, R, RM, D + 1>(X, TI, XA, TIA, q, l, c, omega, dt, sca, rv, i0, i1, valid, r, tIr, tIAr, held);
+  } else if (q < 9 && valid) {
+#pragma unroll
+    for (int h = 0; h < kRecvHeld; h++)
+      if (i0 + h < i1)
+        for (int j = 0; j < rv.nSamples; j++) {
+          double cf = 1.0, v = held[h][0];
+#pragma unroll
+          for (int k = 1; k < O; k++) {
+            cf *= rv.tau[j] / k;
+            v += cf * held[h][k];
+          }
+          rv.buf[((int64_t(i0 + h) * rv.maxBuf + rv.slot[j]) * 9 + q) * R + r] = v;
+        }
   }
 }
 
 // (step.cuh)
-constexpr int kFacLen = 540;
 template <typename T, int O, int R>
 struct SGeo;
 template <typename T, int O, int R>
 __device__ __forceinline__ void liftRow(const StepArgs<T> &a, const T *in, T *wt, int t, int l, int64_t e, int r,
                                         bool valid);
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 __device__ __forceinline__ const T *facPtr(const T *fac, int64_t e);
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 struct FacU;
 template <typename T, int O, int R, typename Z>
 __device__ __forceinline__ void liftApply(const T *wt, const Z &U, int l, T *acc);
@@ -2044,20 +2067,23 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
   T zero[B];
 #pragma unroll
   for (int n = 0; n < B; n++) zero[n] = T(0);
+  // pending characteristics of a strong-form step complete the rows first (their tile lies over X and
+  // TI, which are written only after every warp has read it)
+  T v[B];
   if (q < 9) {
-    T v[B];
     ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, ev, 9, q, r), v, valid);
-    // pending characteristics of a strong-form step complete the rows first (their tile lies over
-    // X and TI, which are written only after every warp has read it)
-    if constexpr (RM == 0)
-      if (a.faceIn) {
-        static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
-        liftRow<T, O, R>(a, a.faceIn, X, q, l, ev, r, valid);
-        if (q < 3) liftRow<T, O, R>(a, a.faceIn, X, q + 9, l, ev, r, valid);
-        __syncthreads();
-        liftApply<T, O, R>(X, FacU<T, O, R>{facPtr<T, O, R>(a.fac, ev), q}, l, v);
-        __syncthreads();
-      }
+  } else {
+#pragma unroll
+    for (int n = 0; n < B; n++) v[n] = T(0);
+  }
+  if (a.faceIn) {
+    static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
+    for (int t = q; t < 12; t += G::NW) liftRow<T, O, R>(a, a.faceIn, X, t, l, ev, r, valid);
+    __syncthreads();
+    liftApply<T, O, R>(X, FacU<T, O, R, RM>{facPtr<T, O, R, RM>(a.fac, ev), q}, l, v);
+    __syncthreads();
+  }
+  if (q < 9) {
     stRow<T, B>(rowPtr<T, SB>(X, q, l), v);
     if constexpr (G::tiSmem)
       stRow<T, B>(rowPtr<T, SB>(TI, q, l), zero);
@@ -2069,9 +2095,14 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
     const int s = q - 9;
 #pragma unroll
     for (int m = 0; m < RM; m++) {
-      T v[B];
-      ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsA, ev, RM * 6, m * 6 + s, r), v, valid);
-      stRow<T, B>(rowPtr<T, SB>(XA, m * 6 + s, l), v);
+      T va[B];
+      ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsA, ev, RM * 6, m * 6 + s, r), va, valid);
+      if (a.faceIn) {
+        const T om = T(a.omega[m]);
+#pragma unroll
+        for (int n = 0; n < B; n++) va[n] = fmaT(om, v[n], va[n]);
+      }
+      stRow<T, B>(rowPtr<T, SB>(XA, m * 6 + s, l), va);
       if constexpr (G::tiSmem)
         stRow<T, B>(rowPtr<T, SB>(TIA, m * 6 + s, l), zero);
       else {
@@ -2084,7 +2115,8 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
   c.load(a, ev, valid, q);
   __syncthreads();
   const int i0 = valid ? rv.grpOff[grp] : 0, i1 = valid ? rv.grpOff[grp + 1] : 0;
-  recvAll<T, O, R, RM, 0>(X, TI, XA, TIA, q, l, c, a.omega, dt, dt, rv, i0, i1, valid, r, tIr, tIAr);
+  double held[kRecvHeld][O];
+  recvAll<T, O, R, RM, 0>(X, TI, XA, TIA, q, l, c, a.omega, dt, dt, rv, i0, i1, valid, r, tIr, tIAr, held);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2110,6 +2142,8 @@ struct SrcArgs {
   int64_t step = 0;
   // sources in elements at or beyond elLimit (not stepped) are skipped
   int64_t elLimit = 0x7fffffffffffffffLL;
+  // the integrals of this step's sources computed ahead (kSrcIntegrals), or null: here
+  const double *amp = nullptr;
 };
 
 __device__ inline double seriesIntegral(double dx, double xStart, int64_t nPts, const double *vals, double x1,
@@ -2153,7 +2187,8 @@ __global__ void kSources(T *dofsE, SrcArgs s) {
     for (int i = s.grpOff[g]; i < s.grpOff[g + 1]; i++) {
       const double a1 = s.clk0 ? s.clk0[i] + k * s.clkDt[i] : t1;
       const double a2 = s.clk0 ? a1 + s.clkDt[i] : t1 + s.dt;
-      const double in = seriesIntegral(s.dts[i], s.t0[i], s.nPts[i], s.ts + s.tsOff[i], a1, a2, s.tol);
+      const double in =
+          s.amp ? s.amp[i] : seriesIntegral(s.dts[i], s.t0[i], s.nPts[i], s.ts + s.tsOff[i], a1, a2, s.tol);
       const double sc = in * s.scal[i * 9 + q];
       T *p = dofsE + ((s.el[i] * 9 + q) * R + s.run[i]) * int64_t(padGlobal<T>(B)) + md;
       *p = T(double(*p) + sc * s.bEval[i * B + md]);

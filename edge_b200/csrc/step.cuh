@@ -26,14 +26,20 @@
 
 namespace edge_b200 {
 
-// coefficients of an element (kBuildStep), in the kernel's precision: U [4][9][4] (three values and
-// a zero), star rows [9][12] (derivative direction d, slot i at 3 d + i), then [4][9][8]: V0[i][0..2],
-// the neighbour's V1[i][0..2] and two zeros. The 16-byte chunks of the E = 32 / R elements of a kernel
-// group are interleaved ([element / E][chunk][E][W]), so that a warp's lanes load consecutive chunks
-// (with one run per lane's element, a chunk at an element's stride would take a cache line per lane:
-// 32 instead of 4 wavefronts a load).
-constexpr int kFacU = 0, kFacStar = 144, kFacV = 252;
-static_assert(kFacLen == kFacV + 288, "coefficient layout");
+// Coefficients of an element (kBuildStep), in the kernel's precision: U [4][9 or 15][4] (three values
+// and a zero; with attenuation the anelastic stress rows follow the nine elastic ones), star rows
+// [9][12] (derivative direction d, slot i at 3 d + i), with attenuation the anelastic star rows [6][8]
+// (2 d + i) and source matrices [RM][12], then [4][9][8]: V0[i][0..2], the neighbour's V1[i][0..2] and
+// two zeros. The 16-byte chunks of the E = 32 / R elements of a kernel group are interleaved
+// ([element / E][chunk][E][W]), so that a warp's lanes load consecutive chunks (with one run per
+// lane's element, a chunk at an element's stride would take a cache line per lane: 32 instead of 4
+// wavefronts a load).
+template <int RM>
+struct FacL {
+  static constexpr int rows = 9 + (RM ? 6 : 0);
+  static constexpr int U = 0, star = 16 * rows, starA = star + 108, src = starA + (RM ? 48 : 0),
+                       V = src + 12 * RM, len = V + 288;
+};
 constexpr uint32_t kNoNeighbour = 0xffffffffu;
 
 template <typename T, int O, int R>
@@ -71,7 +77,7 @@ struct SGeo {
   static constexpr size_t offC = offD + (dofTile ? nX * sizeof(T) : 0);
   // coefficients by cp.async a group ahead: U and the star rows, and the V rows, each where they
   // fit (with few runs per element they are read straight from global memory instead)
-  static constexpr size_t bytesU = size_t(E) * kFacV * sizeof(T), bytesV = size_t(E) * (kFacLen - kFacV) * sizeof(T);
+  static constexpr size_t bytesU = size_t(E) * FacL<0>::V * sizeof(T), bytesV = size_t(E) * (FacL<0>::len - FacL<0>::V) * sizeof(T);
   static constexpr bool smemU = E <= 4 && offC + bytesU <= budget;
   static constexpr bool smemV = smemU && offC + bytesU + bytesV <= budget;
   static constexpr size_t offV = offC + (smemU ? bytesU : 0);
@@ -276,10 +282,10 @@ __device__ __forceinline__ void liftPair(const T *wt, const T *u2, const T *u3, 
 }
 // coefficients of element e (its first chunk): in device memory, and n values at offset `off` of it
 // or of the same layout in shared memory
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 __device__ __forceinline__ const T *facPtr(const T *fac, int64_t e) {
   using G = SGeo<T, O, R>;
-  return fac + (e / G::E) * (kFacLen * G::E) + (e % G::E) * G::W;
+  return fac + (e / G::E) * (FacL<RM>::len * G::E) + (e % G::E) * G::W;
 }
 template <int N, typename T, int O, int R>
 __device__ __forceinline__ void ldFac(const T *p, int off, T *v) {
@@ -289,11 +295,11 @@ __device__ __forceinline__ void ldFac(const T *p, int off, T *v) {
 }
 // U of row q per face: read where it is used (shared memory; rare launches), or held in registers
 // since the start of the group (device memory)
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 struct FacU {
   const T *p;
   int q;
-  __device__ __forceinline__ void operator()(int f, T (&u)[4]) const { ldFac<4, T, O, R>(p, kFacU + f * 36 + q * 4, u); }
+  __device__ __forceinline__ void operator()(int f, T (&u)[4]) const { ldFac<4, T, O, R>(p, FacL<RM>::U + f * (4 * FacL<RM>::rows) + q * 4, u); }
 };
 template <typename T>
 struct RegU {
@@ -318,31 +324,32 @@ __device__ __forceinline__ void liftApply(const T *wt, const Z &U, int l, T *acc
 }
 
 // cp.async of coefficients [from, to) of group g's elements into buf, in the same layout
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 __device__ __forceinline__ void issueFac(const StepArgs<T> &a, T *buf, int from, int to, int64_t g, int64_t nGroups) {
   using G = SGeo<T, O, R>;
   if (g >= nGroups) return;
   const int n = (to - from) / G::W * G::E;
-  for (int i = threadIdx.x; i < n; i += G::NT) {
+  for (int i = threadIdx.x; i < n; i += 32 * FacL<RM>::rows) {
     const int eo = i % G::E;
     if (g * G::E + eo >= a.elCount) continue;
-    cpAsync16(buf + i * G::W, facPtr<T, O, R>(a.fac, a.elFirst + g * G::E + eo) + (from + i / G::E * G::W) * G::E);
+    cpAsync16(buf + i * G::W, facPtr<T, O, R, RM>(a.fac, a.elFirst + g * G::E + eo) + (from + i / G::E * G::W) * G::E);
   }
 }
 // the same coefficients into L2 (a group ahead, where the kernel reads them from device memory)
-template <typename T, int O, int R>
+template <typename T, int O, int R, int RM>
 __device__ __forceinline__ void prefetchFac(const StepArgs<T> &a, int from, int to, int64_t g, int64_t nGroups) {
   using G = SGeo<T, O, R>;
   if (g >= nGroups) return;
-  const char *p = reinterpret_cast<const char *>(a.fac + ((a.elFirst + g * G::E) / G::E * kFacLen + from) * G::E);
+  const char *p = reinterpret_cast<const char *>(a.fac + ((a.elFirst + g * G::E) / G::E * FacL<RM>::len + from) * G::E);
   const int bytes = (to - from) * G::E * int(sizeof(T));
-  for (int i = threadIdx.x * 128; i < bytes; i += G::NT * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+  for (int i = threadIdx.x * 128; i < bytes; i += 32 * FacL<RM>::rows * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
 }
 
 // DOF rows of a group between device memory and the tile rows of warp q: with one run per element
 // consecutive lanes move the consecutive chunks of an element's row (a row per lane would touch a
 // cache line per lane), with more runs those of an element's runs. nv: elements of the group.
-template <typename T, int O, int R, int S>
+// row: of the nRows of the DOF array and its tile
+template <typename T, int O, int R, int S, int NR = 9>
 __device__ __forceinline__ void rowsIn(T *tile, const T *dofs, int64_t e0, int nv, int q, int l) {
   using G = SGeo<T, O, R>;
   if constexpr (R == 1) {
@@ -350,13 +357,13 @@ __device__ __forceinline__ void rowsIn(T *tile, const T *dofs, int64_t e0, int n
 #pragma unroll
     for (int it = 0; it < C; it++) {
       const int k = it * 32 + l, eo = k / C, c = k - eo * C;
-      if (eo < nv) cpAsync16(tile + (q * 32 + eo) * S + c * G::W, dofs + ((e0 + eo) * 9 + q) * G::GB + c * G::W);
+      if (eo < nv) cpAsync16(tile + (q * 32 + eo) * S + c * G::W, dofs + ((e0 + eo) * NR + q) * G::GB + c * G::W);
     }
   } else {
-    if (l / R < nv) copyDofRows<T, R, G::GB, S>(tile, dofs, e0 + l / R, q, l / R, l % R);
+    if (l / R < nv) copyRows<T, R, G::GB, S>(tile, dofs, e0 + l / R, NR, q, l / R, l % R);
   }
 }
-template <typename T, int O, int R, int S>
+template <typename T, int O, int R, int S, int NR = 9>
 __device__ __forceinline__ void rowsOut(const T *tile, T *dofs, int64_t e0, int nv, int q, int l) {
   using G = SGeo<T, O, R>;
   if constexpr (R == 1) {
@@ -366,11 +373,11 @@ __device__ __forceinline__ void rowsOut(const T *tile, T *dofs, int64_t e0, int 
       const int k = it * 32 + l, eo = k / C, c = k - eo * C;
       T v[G::W];
       ldChunk<T>(tile + (q * 32 + eo) * S + c * G::W, v);
-      if (eo < nv) stChunk<T>(dofs + ((e0 + eo) * 9 + q) * G::GB + c * G::W, v);
+      if (eo < nv) stChunk<T>(dofs + ((e0 + eo) * NR + q) * G::GB + c * G::W, v);
     }
   } else {
     if (l / R < nv)
-      storeRowsCoalesced<T, R, G::GB, S>(tile, dofs + ((e0 + l / R) * 9 + q) * int64_t(R * G::GB), q, l / R, l % R);
+      storeRowsCoalesced<T, R, G::GB, S>(tile, dofs + ((e0 + l / R) * NR + q) * int64_t(R * G::GB), q, l / R, l % R);
   }
 }
 
@@ -489,7 +496,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     const int eo = l / R, r = l % R;
     const int64_t g = blockIdx.x;
     if constexpr (G::dofTile) rowsIn<T, O, R, SB>(D, a.dofsE, a.elFirst + g * E, inGroup(g), q, l);
-    if constexpr (G::smemU) issueFac<T, O, R>(a, bufU, 0, kFacV, g, nGroups);
+    if constexpr (G::smemU) issueFac<T, O, R, 0>(a, bufU, 0, FacL<0>::V, g, nGroups);
     // pending characteristics: warp q takes rows q and (q < 3) q + 9; gather entries and own parts of
     // the current group
     const int t1 = q < 3 ? q + 9 : q;
@@ -517,17 +524,17 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     const int64_t e = valid ? a.elFirst + g * E + eo : a.elFirst;
     const int64_t gn = g + gridDim.x;
     const T dt = a.grpDt ? T(a.grpDt[g]) : dt0;
-    const T *const facE = facPtr<T, O, R>(a.fac, e);
+    const T *const facE = facPtr<T, O, R, 0>(a.fac, e);
     const T *const cU = G::smemU ? bufU + eo * G::W : facE;
-    const T *const cV = G::smemV ? bufV + eo * G::W : facE + kFacV * E;
+    const T *const cV = G::smemV ? bufV + eo * G::W : facE + FacL<0>::V * E;
     // U and star rows: read where they are used from shared memory, from here on from device memory
     RegU<T> ru;
     T st[12];
-    const FacU<T, O, R> su{cU, q};
+    const FacU<T, O, R, 0> su{cU, q};
     if constexpr (!G::smemU) {
 #pragma unroll
       for (int f = 0; f < 4; f++) su(f, ru.u[f]);
-      ldFac<12, T, O, R>(cU, kFacStar + q * 12, st);
+      ldFac<12, T, O, R>(cU, FacL<0>::star + q * 12, st);
     }
     // the next group's element of this lane
     const bool validN = gn < nGroups && gn * E + eo < a.elCount;
@@ -545,7 +552,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     }
     __syncthreads();
     // every warp is past the previous group's characteristics, the last readers of V and of X
-    if constexpr (G::smemV) issueFac<T, O, R>(a, bufV, kFacV, kFacLen, g, nGroups);
+    if constexpr (G::smemV) issueFac<T, O, R, 0>(a, bufV, FacL<0>::V, FacL<0>::len, g, nGroups);
     cpAsyncCommit();
     T acc[B];
     if constexpr (G::dofTile) {
@@ -560,7 +567,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
         liftApply<T, O, R>(XP, ru, l, acc);
     }
     stRow<T, B>(rowPtr<T, SB>(X, q, l), acc);
-    if constexpr (G::smemU) ldFac<12, T, O, R>(cU, kFacStar + q * 12, st);
+    if constexpr (G::smemU) ldFac<12, T, O, R>(cU, FacL<0>::star + q * 12, st);
     int cols[3];
     T cs[3][3];
 #pragma unroll
@@ -571,8 +578,8 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     }
     __syncthreads();
     // every thread read this group's U and star rows
-    if constexpr (G::smemU) issueFac<T, O, R>(a, bufU, 0, kFacV, gn, nGroups);
-    if constexpr (!G::smemV) prefetchFac<T, O, R>(a, G::smemU ? kFacV : 0, kFacLen, gn, nGroups);
+    if constexpr (G::smemU) issueFac<T, O, R, 0>(a, bufU, 0, FacL<0>::V, gn, nGroups);
+    if constexpr (!G::smemV) prefetchFac<T, O, R, 0>(a, G::smemU ? FacL<0>::V : 0, FacL<0>::len, gn, nGroups);
     cpAsyncCommit();
     T ti[G::NK];
     ckStrong<T, O, R, 1>(X, XP, q, l, cols, cs, dt, dt, acc, ti);
@@ -652,9 +659,9 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctasLift) kL
     const int64_t e = valid ? a.elFirst + g * E + eo : a.elFirst;
     const int nv = int(min(a.elCount - g * E, int64_t(E)));
     if constexpr (G::liftTile) rowsIn<T, O, R, SB>(D, a.dofsE, a.elFirst + g * E, nv, q, l);
-    if constexpr (G::smemU) issueFac<T, O, R>(a, bufU, 0, kFacV, g, nGroups);
+    if constexpr (G::smemU) issueFac<T, O, R, 0>(a, bufU, 0, FacL<0>::V, g, nGroups);
     cpAsyncCommit();
-    const FacU<T, O, R> su{G::smemU ? bufU + eo * G::W : facPtr<T, O, R>(a.fac, e), q};
+    const FacU<T, O, R, 0> su{G::smemU ? bufU + eo * G::W : facPtr<T, O, R, 0>(a.fac, e), q};
     RegU<T> ru;
     if constexpr (!G::smemU) {
 #pragma unroll

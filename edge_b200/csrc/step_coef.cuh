@@ -1,73 +1,34 @@
-// Coefficients of the strong-form step (step.cuh) from the caller's star matrices, flux solvers and
-// connectivity: per element U, star rows and V rows (kFacLen values), and the gather table.
+// Coefficients of the strong-form step (step.cuh, step_visc.cuh) from the caller's star matrices, flux
+// solvers and connectivity: per element U, star rows, anelastic coefficients and V rows (FacL), and the
+// gather table.
 #pragma once
-#include "step.cuh"
+#include "step_visc.cuh"
 
 namespace edge_b200 {
 
-// Orthonormal basis Q (3 x 9) of the rows of S (9 x 9) by Gram-Schmidt with pivoting, each direction
-// orthogonalised twice; a direction without a row left is zero. Returns the largest squared norm
-// that a row keeps outside Q. S is overwritten.
-__device__ __forceinline__ double rowBasis(double (&S)[9][9], double (&Q)[3][9]) {
-  for (int k = 0; k < 3; k++) {
-    double best = 0, v[9];
+// Nine lanes share a face, lane a its row a of the 9 x 9 solvers; what they exchange goes through this
+// (a thread per face keeps its matrices in local memory: 6.2 against 0.6 ms for 72,864 elements).
+struct FaceTeam {
+  double S[9][9], N[9][9], U[9][3], V0[9][3], red[9];
+};
+constexpr int kTeams = 3;          // per warp
+constexpr int kBuildWarps = 4;     // per block
+constexpr double kRankTol2 = 1e-18;  // squared share of a scaled row outside three directions
+
+__device__ __forceinline__ double teamMax(FaceTeam &t, int a, double v, int from, int to) {
+  __syncwarp();
+  t.red[a] = v;
+  __syncwarp();
+  double m = 0;
 #pragma unroll
-    for (int j = 0; j < 9; j++) v[j] = 0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-      double n2 = 0;
-#pragma unroll
-      for (int j = 0; j < 9; j++) n2 += S[i][j] * S[i][j];
-      if (n2 > best) {
-        best = n2;
-#pragma unroll
-        for (int j = 0; j < 9; j++) v[j] = S[i][j];
-      }
-    }
-    for (int pass = 0; pass < 2; pass++)
-#pragma unroll
-      for (int kk = 0; kk < 3; kk++)
-        if (kk < k) {
-          double d = 0;
-#pragma unroll
-          for (int j = 0; j < 9; j++) d += v[j] * Q[kk][j];
-#pragma unroll
-          for (int j = 0; j < 9; j++) v[j] -= d * Q[kk][j];
-        }
-    double n2 = 0;
-#pragma unroll
-    for (int j = 0; j < 9; j++) n2 += v[j] * v[j];
-    // rows of unit scale: what rounding leaves of a dependent row is no direction
-    const double inv = n2 > 1e-24 ? 1.0 / sqrt(n2) : 0.0;
-#pragma unroll
-    for (int kk = 0; kk < 3; kk++)
-      if (kk == k)
-#pragma unroll
-        for (int j = 0; j < 9; j++) Q[kk][j] = v[j] * inv;
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-      double d = 0;
-#pragma unroll
-      for (int j = 0; j < 9; j++) d += S[i][j] * v[j];
-      d *= inv * inv;
-#pragma unroll
-      for (int j = 0; j < 9; j++) S[i][j] -= d * v[j];
-    }
-  }
-  double res = 0;
-#pragma unroll
-  for (int i = 0; i < 9; i++) {
-    double n2 = 0;
-#pragma unroll
-    for (int j = 0; j < 9; j++) n2 += S[i][j] * S[i][j];
-    res = n2 > res ? n2 : res;
-  }
-  return res;
+  for (int i = 0; i < 9; i++)
+    if (i >= from && i < to) m = fmax(m, t.red[i]);
+  return m;
 }
 
 // Row and column scales of a flux solver, one for the stresses and one for the velocities (as
-// inputs and as outputs they differ by the moduli and impedances): S = M_ij / (r_i c_j) with entries
-// of at most one. (A scale per row or column would blow up the rounding of those that vanish; the
+// inputs and as outputs they differ by the moduli and impedances): M_ij / (r_i c_j) has entries of
+// at most one. (A scale per row or column would blow up the rounding of those that vanish; the
 // scales of a face without a neighbour are those of fsE[0], before a free surface's velocity
 // columns cancel.)
 struct Scales {
@@ -75,165 +36,188 @@ struct Scales {
   __device__ __forceinline__ double r(int i) const { return i < 6 ? rS : rV; }
   __device__ __forceinline__ double c(int j) const { return j < 6 ? cS : cV; }
 };
-__device__ __forceinline__ Scales scales(const double (&M)[9][9]) {
-  Scales s{0, 0, 0, 0};
+__device__ __forceinline__ Scales scales(FaceTeam &t, int a, const double (&M)[9]) {
+  double mS = 0, mV = 0;
 #pragma unroll
-  for (int i = 0; i < 9; i++)
-#pragma unroll
-    for (int j = 0; j < 9; j++) {
-      if (i < 6)
-        s.rS = fmax(s.rS, fabs(M[i][j]));
-      else
-        s.rV = fmax(s.rV, fabs(M[i][j]));
-    }
+  for (int j = 0; j < 9; j++) (j < 6 ? mS : mV) = fmax(j < 6 ? mS : mV, fabs(M[j]));
+  Scales s;
+  s.rS = teamMax(t, a, fmax(mS, mV), 0, 6);
+  s.rV = teamMax(t, a, fmax(mS, mV), 6, 9);
   if (!(s.rS > 0)) s.rS = 1.0;
   if (!(s.rV > 0)) s.rV = 1.0;
-#pragma unroll
-  for (int i = 0; i < 9; i++)
-#pragma unroll
-    for (int j = 0; j < 9; j++) {
-      if (j < 6)
-        s.cS = fmax(s.cS, fabs(M[i][j]) / s.r(i));
-      else
-        s.cV = fmax(s.cV, fabs(M[i][j]) / s.r(i));
-    }
+  s.cS = teamMax(t, a, mS / s.r(a), 0, 9);
+  s.cV = teamMax(t, a, mV / s.r(a), 0, 9);
   if (!(s.cS > 0)) s.cS = 1.0;
   if (!(s.cV > 0)) s.cV = 1.0;
   return s;
 }
 
-__device__ __forceinline__ void load81(const double *p, double (&M)[9][9]) {
+// Orthonormal basis Q (3 x 9, in every lane) of the rows of the scaled solver, this lane's row S, by
+// Gram-Schmidt with pivoting, each direction orthogonalised twice; a direction without a row left is
+// zero. Returns what this lane's row keeps outside Q (squared norm).
+__device__ __forceinline__ double rowBasis(FaceTeam &t, int a, double (&S)[9], double (&Q)[3][9]) {
 #pragma unroll
-  for (int i = 0; i < 9; i++)
+  for (int k = 0; k < 3; k++) {
+    double n2 = 0;
+    __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 9; j++) M[i][j] = __ldg(p + i * 9 + j);
+    for (int j = 0; j < 9; j++) {
+      n2 += S[j] * S[j];
+      t.S[a][j] = S[j];
+    }
+    t.red[a] = n2;
+    __syncwarp();
+    int piv = 0;
+    double best = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++)
+      if (t.red[i] > best) {
+        best = t.red[i];
+        piv = i;
+      }
+    double v[9];
+#pragma unroll
+    for (int j = 0; j < 9; j++) v[j] = best > 0 ? t.S[piv][j] : 0.0;
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+      for (int kk = 0; kk < k; kk++) {
+        double d = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) d += v[j] * Q[kk][j];
+#pragma unroll
+        for (int j = 0; j < 9; j++) v[j] -= d * Q[kk][j];
+      }
+    double l2 = 0;
+#pragma unroll
+    for (int j = 0; j < 9; j++) l2 += v[j] * v[j];
+    // rows of unit scale: what rounding leaves of a dependent row is no direction
+    const double inv = l2 > 1e-24 ? 1.0 / sqrt(l2) : 0.0;
+    double d = 0;
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+      Q[k][j] = v[j] * inv;
+      d += S[j] * Q[k][j];
+    }
+#pragma unroll
+    for (int j = 0; j < 9; j++) S[j] -= d * Q[k][j];
+  }
+  double res = 0;
+#pragma unroll
+  for (int j = 0; j < 9; j++) res += S[j] * S[j];
+  return res;
 }
 
-constexpr double kRankTol2 = 1e-18;  // squared share of a scaled row outside three directions
-
-// One face per thread, part 0: V1 of the face's reader (a function of the reader's fsE[1] alone, so
-// that parts of a partition agree on it); part 1: U and V0 of the face. Counts faces whose flux
-// solvers are not of rank 3 in this form in *bad.
+// Two items per face: part 0: V1 of the face's reader (a function of the reader's fsE[1] alone, so that
+// parts of a partition agree on it); part 1: U and V0 of the face, and with face 0 the element's other
+// coefficients. Counts lanes that find their face's solvers not of rank 3 in this form in *bad.
 template <typename T>
-__global__ void __launch_bounds__(64) kBuildStep(const double *fsE, const double *starE, const int32_t *elFaEl,
-                                                 const uint8_t *fId, const uint8_t *vId, const uint8_t *faType,
-                                                 int64_t nEl, int order, int E, T *fac, uint32_t *gath, int *bad) {
-  const int64_t total = (nEl * 4 + 31) / 32 * 64;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    // neighbouring threads take the same part
-    const int part = int((i >> 5) & 1);
-    const int64_t ef = (i >> 6) * 32 + (i & 31);
-    if (ef >= nEl * 4) continue;
-    const int64_t e = ef >> 2;
+__global__ void __launch_bounds__(kBuildWarps * 32)
+    kBuildStep(const double *fsE, const double *starE, const double *fsA, const double *starA, const double *srcA,
+               int rm, const int32_t *elFaEl, const uint8_t *fId, const uint8_t *vId, const uint8_t *faType,
+               int64_t nEl, int order, int E, T *fac, uint32_t *gath, int *bad) {
+  __shared__ FaceTeam teams[kBuildWarps][kTeams + 1];
+  const int l = threadIdx.x & 31, team = l / 9, a = l - 9 * team;  // (lanes 27 .. 31 repeat the last team's item)
+  FaceTeam &t = teams[threadIdx.x >> 5][team];
+  const int64_t items = nEl * 8, stride = int64_t(gridDim.x) * kBuildWarps * kTeams;
+  for (int64_t i0 = (int64_t(blockIdx.x) * kBuildWarps + (threadIdx.x >> 5)) * kTeams; i0 < items; i0 += stride) {
+    const int64_t i = min(i0 + min(team, kTeams - 1), items - 1);
+    const bool mine = team < kTeams && i0 + team < items;
+    const int part = int(i & 1);
+    const int64_t ef = i >> 1, e = ef >> 2;
     const int f = int(ef & 3), ty = faType[ef];
-    // value i of the element's coefficients (16-byte chunks interleaved over E elements)
+    // value k of the element's coefficients (16-byte chunks interleaved over E elements)
     constexpr int W = 16 / int(sizeof(T));
-    T *const fe = fac + (e / E) * (int64_t(kFacLen) * E) + (e % E) * W;
-    const auto put = [&](int i, double v) { fe[i / W * (E * W) + i % W] = T(v); };
-    const int V = kFacV + f * 72;
-    double M[9][9], Q[3][9];
-    if (part == 0) {
-      // (the neighbour reads this element's projection at its own face: its fsE[1] there)
-      gath[ef] = kNoNeighbour;
-      if (ty != FT_INNER) {
+    const int rows = rm ? FacL<3>::rows : FacL<0>::rows, oStar = rm ? FacL<3>::star : FacL<0>::star;
+    const int V = (rm ? FacL<3>::src + 12 * rm : FacL<0>::V) + f * 72;
+    const int len = V - f * 72 + 288;
+    T *const fe = fac + (e / E) * (int64_t(len) * E) + (e % E) * W;
+    const auto put = [&](int k, double v) {
+      if (mine) fe[k / W * (E * W) + k % W] = T(v);
+    };
+    const bool inner = ty == FT_INNER;
+    const int64_t n = inner ? elFaEl[ef] : e;
+    const int fo = inner ? fId[ef] : f;
+    // this lane's rows: M what the basis comes from, N the own side
+    // (part 0: the neighbour reads this element's projection at its own face, through its fsE[1] there)
+    const double *pm = fsE + (nEl * 4 + (part == 0 ? n * 4 + fo : ef)) * 81 + a * 9;
+    const double *pn = fsE + ef * 81 + a * 9;
+    double M[9], N[9], add[9];
 #pragma unroll
-        for (int j = 0; j < 9; j++) {
-          for (int k = 3; k < 8; k++) put(V + 8 * j + k, 0);
-        }
-        continue;
-      }
-      const int64_t n = elFaEl[ef];
-      const int fo = fId[ef];
-      gath[ef] = uint32_t((n * 4 + fo) * 4 + kFacePerm[order - 2][fo][f][vId[ef]]);
-      load81(fsE + ((nEl + n) * 4 + fo) * 81, M);
-      const Scales sc = scales(M);
-#pragma unroll
-      for (int a = 0; a < 9; a++)
-#pragma unroll
-        for (int j = 0; j < 9; j++) M[a][j] /= sc.r(a) * sc.c(j);
-      if (rowBasis(M, Q) > kRankTol2) atomicAdd(bad, 1);
-#pragma unroll
-      for (int j = 0; j < 9; j++) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) put(V + 8 * j + 3 + k, sc.c(j) * Q[k][j]);
-        put(V + 8 * j + 6, 0);
-        put(V + 8 * j + 7, 0);
-      }
-      continue;
+    for (int j = 0; j < 9; j++) {
+      M[j] = __ldg(pm + j);
+      N[j] = __ldg(pn + j);
+      add[j] = 0;
     }
-    // own side: N = fsE[0] + sum_d n_fd star_d (+ fsE[1] of a free surface, which reads this element)
-    double N[9][9];
-    load81(fsE + ef * 81, N);
-    Scales sc = scales(N);
-    const double n0 = f == 2 ? -1.0 : f == 3 ? 1.0 : 0.0, n1 = f == 1 ? -1.0 : f == 3 ? 1.0 : 0.0,
-                 n2 = f == 0 ? -1.0 : f == 3 ? 1.0 : 0.0;
-    const double *st = starE + e * 72;
-#pragma unroll
-    for (int q = 0; q < 9; q++) {
+    const Scales sc0 = scales(t, a, N), sc1 = scales(t, a, M);
+    const Scales sc = inner ? sc1 : sc0;
+    const double nrm[3] = {f == 2 ? -1.0 : f == 3 ? 1.0 : 0.0, f == 1 ? -1.0 : f == 3 ? 1.0 : 0.0,
+                           f == 0 ? -1.0 : f == 3 ? 1.0 : 0.0};
+    if (part == 1) {
+      // N = fsE[0] + sum_d n_fd star_d (+ fsE[1] of a free surface, which reads this element)
+      const double *st = starE + e * 72;
       double sd[3][3];
 #pragma unroll
       for (int s = 0; s < 3; s++) {
-        const int idx = kStarIdx[q][s], col = kStarCol[q][s];
+        const int idx = kStarIdx[a][s], col = kStarCol[a][s];
         double v[3] = {0, 0, 0};
         if (idx >= 0)
 #pragma unroll
           for (int d = 0; d < 3; d++) v[d] = __ldg(st + d * 24 + idx);
-        const double add = n0 * v[0] + n1 * v[1] + n2 * v[2];
 #pragma unroll
         for (int j = 0; j < 9; j++)
-          if (j == col) N[q][j] += add;
+          if (j == col) add[j] += nrm[0] * v[0] + nrm[1] * v[1] + nrm[2] * v[2];
 #pragma unroll
         for (int d = 0; d < 3; d++) sd[d][s] = kStarDir[0][d] * v[0] + kStarDir[1][d] * v[1] + kStarDir[2][d] * v[2];
       }
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        N[j] += add[j];
+        if (ty == FT_FREE) N[j] += M[j];
+        if (!inner) M[j] = N[j];
+      }
       if (f == 0) {
         // the star rows along the derivative directions of the generated products
-        const int o = kFacStar + q * 12;
 #pragma unroll
-        for (int d = 0; d < 3; d++)
-#pragma unroll
-          for (int s = 0; s < 3; s++) put(o + 3 * d + s, sd[d][s]);
-#pragma unroll
-        for (int s = 9; s < 12; s++) put(o + s, 0);
+        for (int k = 0; k < 12; k++) put(oStar + a * 12 + k, k < 9 ? sd[k < 9 ? k / 3 : 0][k % 3] : 0.0);
       }
+    } else if (mine && a == 0) {
+      gath[ef] = inner ? uint32_t((n * 4 + fo) * 4 + kFacePerm[order - 2][fo][f][vId[ef]]) : kNoNeighbour;
     }
-    if (ty == FT_INNER) {
-      load81(fsE + (nEl * 4 + ef) * 81, M);
-      sc = scales(M);
-    } else {
-      if (ty == FT_FREE) {
-        load81(fsE + (nEl * 4 + ef) * 81, M);
+    double S[9], Q[3][9];
 #pragma unroll
-        for (int a = 0; a < 9; a++)
+    for (int j = 0; j < 9; j++) S[j] = M[j] = M[j] / (sc.r(a) * sc.c(j));
+    bool off = rowBasis(t, a, S, Q) > kRankTol2;
+    if (part == 0) {
 #pragma unroll
-          for (int j = 0; j < 9; j++) N[a][j] += M[a][j];
-      }
+      for (int j = 0; j < 9; j++)
+        if (j == a) {
 #pragma unroll
-      for (int a = 0; a < 9; a++)
-#pragma unroll
-        for (int j = 0; j < 9; j++) M[a][j] = N[a][j];
+          for (int k = 0; k < 3; k++) put(V + 8 * j + 3 + k, inner ? sc.c(j) * Q[k][j] : 0.0);
+          put(V + 8 * j + 6, 0);
+          put(V + 8 * j + 7, 0);
+        }
+      off = off && inner;
     }
-    double S[9][9];
+    // U (scaled rows), then V0 from U V0^T = N: every lane holds U and solves for its own column
 #pragma unroll
-    for (int a = 0; a < 9; a++)
+    for (int k = 0; k < 3; k++) {
+      double u = 0;
 #pragma unroll
-      for (int j = 0; j < 9; j++) S[a][j] = M[a][j] = M[a][j] / (sc.r(a) * sc.c(j));
-    bool off = rowBasis(S, Q) > kRankTol2;
-    // scaled U = (M / r c) Q^T, its orthonormal columns A = U Rm^-1 (twice)
-    double U[9][3], A[3][9], Rm[3][3];
+      for (int j = 0; j < 9; j++) u += M[j] * Q[k][j];
+      t.U[a][k] = u;
+      if (part == 1) put(f * 4 * rows + a * 4 + k, sc.r(a) * u);
+    }
+    if (part == 1) put(f * 4 * rows + a * 4 + 3, 0);
 #pragma unroll
-    for (int a = 0; a < 9; a++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        double u = 0;
-#pragma unroll
-        for (int j = 0; j < 9; j++) u += M[a][j] * Q[k][j];
-        U[a][k] = u;
-      }
+    for (int j = 0; j < 9; j++) t.N[a][j] = N[j] / sc.r(a);
+    __syncwarp();
+    double A[3][9], Rm[3][3], b[3], x[3], nj[9];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       double v[9];
 #pragma unroll
-      for (int a = 0; a < 9; a++) v[a] = U[a][k];
+      for (int i2 = 0; i2 < 9; i2++) v[i2] = t.U[i2][k];
 #pragma unroll
       for (int kk = 0; kk < 3; kk++) Rm[kk][k] = 0;
 #pragma unroll
@@ -242,60 +226,117 @@ __global__ void __launch_bounds__(64) kBuildStep(const double *fsE, const double
         for (int kk = 0; kk < k; kk++) {
           double d = 0;
 #pragma unroll
-          for (int a = 0; a < 9; a++) d += v[a] * A[kk][a];
+          for (int i2 = 0; i2 < 9; i2++) d += v[i2] * A[kk][i2];
           Rm[kk][k] += d;
 #pragma unroll
-          for (int a = 0; a < 9; a++) v[a] -= d * A[kk][a];
+          for (int i2 = 0; i2 < 9; i2++) v[i2] -= d * A[kk][i2];
         }
-      double n = 0;
+      double l2 = 0;
 #pragma unroll
-      for (int a = 0; a < 9; a++) n += v[a] * v[a];
-      const double len = sqrt(n);
-      Rm[k][k] = len > 1e-12 ? len : 0.0;
+      for (int i2 = 0; i2 < 9; i2++) l2 += v[i2] * v[i2];
+      const double len2 = sqrt(l2), inv = len2 > 1e-12 ? 1.0 / len2 : 0.0;
+      Rm[k][k] = len2 > 1e-12 ? len2 : 0.0;
 #pragma unroll
-      for (int a = 0; a < 9; a++) A[k][a] = len > 1e-12 ? v[a] / len : 0.0;
-    }
-    // V0: U V0^T = N, column by column (residuals against the largest entry of the column's kind)
-#pragma unroll
-    for (int a = 0; a < 9; a++)
-#pragma unroll
-      for (int j = 0; j < 9; j++) N[a][j] /= sc.r(a);
-    const int U0 = kFacU + f * 36;
-#pragma unroll
-    for (int a = 0; a < 9; a++) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) put(U0 + a * 4 + k, sc.r(a) * U[a][k]);
-      put(U0 + a * 4 + 3, 0);
+      for (int i2 = 0; i2 < 9; i2++) A[k][i2] = v[i2] * inv;
     }
 #pragma unroll
-    for (int j = 0; j < 9; j++) {
-      double b[3];
-      const double top = j < 6 ? sc.cS : sc.cV;
+    for (int i2 = 0; i2 < 9; i2++) nj[i2] = t.N[i2][a];
+    double res = 0;
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        b[k] = 0;
+    for (int k = 0; k < 3; k++) {
+      b[k] = 0;
 #pragma unroll
-        for (int a = 0; a < 9; a++) b[k] += A[k][a] * N[a][j];
-      }
-      double res = 0;
-#pragma unroll
-      for (int a = 0; a < 9; a++) {
-        const double d = N[a][j] - A[0][a] * b[0] - A[1][a] * b[1] - A[2][a] * b[2];
-        res += d * d;
-      }
-      off = off || !(res <= kRankTol2 * top * top);
-      double x[3];
-#pragma unroll
-      for (int k = 2; k >= 0; k--) {
-        double t = b[k];
-#pragma unroll
-        for (int kk = k + 1; kk < 3; kk++) t -= Rm[k][kk] * x[kk];
-        x[k] = Rm[k][k] > 0 ? t / Rm[k][k] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < 3; k++) put(V + 8 * j + k, x[k]);
+      for (int i2 = 0; i2 < 9; i2++) b[k] += A[k][i2] * nj[i2];
     }
-    if (off) atomicAdd(bad, 1);
+#pragma unroll
+    for (int i2 = 0; i2 < 9; i2++) {
+      const double d = nj[i2] - A[0][i2] * b[0] - A[1][i2] * b[1] - A[2][i2] * b[2];
+      res += d * d;
+    }
+#pragma unroll
+    for (int k = 2; k >= 0; k--) {
+      double v = b[k];
+#pragma unroll
+      for (int kk = k + 1; kk < 3; kk++) v -= Rm[k][kk] * x[kk];
+      x[k] = Rm[k][k] > 0 ? v / Rm[k][k] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      t.V0[a][k] = x[k];
+      if (part == 1) put(V + 8 * a + k, x[k]);
+    }
+    // residuals against the largest entry of the column's kind
+    const double top = sc.c(a);
+    if (part == 1) off = off || !(res <= kRankTol2 * top * top);
+    __syncwarp();
+    // (the teams of a warp may hold different parts: all of them pass the warp barriers, and part 0
+    // writes nothing here)
+    if (rm) {
+      // anelastic rows (lanes 0 .. 5): UA over the same basis, and the same V0 has to give
+      // fsA[0]' = fsA[0] + sum_d n_fd starA_d
+      const int s = a < 6 ? a : 0;
+      const double *f0 = fsA + ef * 54 + s * 9, *f1 = fsA + (nEl * 4 + ef) * 54 + s * 9, *sa = starA + e * 27;
+      double na[9], ma[9], mS = 0, mV = 0;
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        na[j] = __ldg(f0 + j);
+        ma[j] = __ldg(f1 + j);
+        const double v = fmax(fabs(na[j]), inner ? fabs(ma[j]) : 0.0);
+        if (j < 6)
+          mS = fmax(mS, v);
+        else
+          mV = fmax(mV, v);
+      }
+      const double topS = teamMax(t, a, mS, 0, 6), topV = teamMax(t, a, mV, 0, 6);
+#pragma unroll
+      for (int i2 = 0; i2 < 2; i2++) {
+        const int idx = kStarAIdx[s][i2], col = 6 + kStarACol[s][i2];
+        double v[3] = {0, 0, 0};
+        if (idx >= 0)
+#pragma unroll
+          for (int d = 0; d < 3; d++) v[d] = __ldg(sa + d * 9 + idx);
+#pragma unroll
+        for (int j = 0; j < 9; j++)
+          if (j == col) na[j] += nrm[0] * v[0] + nrm[1] * v[1] + nrm[2] * v[2];
+        if (part == 1 && f == 0 && a < 6)
+#pragma unroll
+          for (int d = 0; d < 3; d++)
+            put(FacL<3>::starA + s * 8 + 2 * d + i2, kStarDir[0][d] * v[0] + kStarDir[1][d] * v[1] + kStarDir[2][d] * v[2]);
+      }
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        if (ty == FT_FREE) na[j] += ma[j];
+        if (!inner) ma[j] = na[j];
+      }
+      if (part == 1 && a < 6) {
+        double u[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          u[k] = 0;
+#pragma unroll
+          for (int j = 0; j < 9; j++) u[k] += ma[j] / sc.c(j) * Q[k][j];
+          put(f * 4 * rows + (9 + s) * 4 + k, u[k]);
+        }
+        put(f * 4 * rows + (9 + s) * 4 + 3, 0);
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+          const double tol = 1e-9 * (j < 6 ? topS : topV);
+          double r1 = ma[j], r0 = na[j];
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            r1 -= u[k] * sc.c(j) * Q[k][j];
+            r0 -= u[k] * t.V0[j][k];
+          }
+          off = off || !(fabs(r1) <= tol) || !(fabs(r0) <= tol);
+        }
+        if (f == 0) {
+          put(FacL<3>::starA + s * 8 + 6, 0);
+          put(FacL<3>::starA + s * 8 + 7, 0);
+          for (int k = s; k < 12 * rm; k += 6) put(FacL<3>::src + k, srcA[e * 12 * rm + k]);
+        }
+      }
+    }
+    if (off && mine) atomicAdd(bad, 1);
   }
 }
 

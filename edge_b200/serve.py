@@ -114,16 +114,16 @@ def element_data_bytes(n_el, rm=0):
 
 
 def pool_bytes(n_el, order, runs, precision, rm=0, shared=False):
-    """Device memory of a pool context (DOF and anelastic rows, two face-projection buffers of the
-    fused steps, staging, the flux-solver pairs of the pre-mixed face projections and, unless
-    borrowed from the mesh's anchor context (shared), the element data)."""
+    """Device memory of a pool context (DOF and anelastic rows, the face buffer, staging, the
+    coefficients of the step and, unless borrowed from the mesh's anchor context (shared), the
+    element data)."""
     p = 8 if precision == 64 else 4
     w = 16 // p
     gb = math.ceil(host.n_modes(order) / w) * w
     gf = math.ceil(host.n_face_modes(order) / w) * w
     nq = 9 + 6 * rm
-    own = n_el * (nq * runs * gb * p * 2 + 2 * 36 * runs * gf * p + nq * host.n_modes(order) * runs * p
-                  + 4 * 2 * 84 * p + 28)
+    own = n_el * (nq * runs * gb * p * 2 + 36 * runs * gf * p + nq * host.n_modes(order) * runs * p
+                  + (720 if rm else 540) * p + 16 + 28)
     return own + (0 if shared else element_data_bytes(n_el, rm))
 
 

@@ -264,7 +264,9 @@ int edge_b200_wavefield(edge_b200_ctx *ctx, float *out);
  * local, sources) or second half (phase 1: neighbour). pack / unpack move the face blocks
  * [9][R][GF] of n face slots (slots[i] = element * 4 + face, a device int32 array) to / from the
  * device buffer out / in ([n] blocks of edge_b200_face_block_bytes each, GF = F rounded up to 16
- * bytes), ordered on the context stream; slots outside the mesh are skipped. Time groups need the
+ * bytes; in the strong form a block holds the three characteristic rows of its face), ordered on the
+ * context stream; slots outside the mesh are skipped. All parts have to take the same form
+ * (edge_b200_step_form). Time groups need the
  * whole mesh owned. To overlap the exchange with work, as the reference's inner / send regions do
  * (src/impl/seismic/setup.inc:337-399), number the owned elements with a face neighbour in another
  * part first and give their count to edge_b200_set_send_count: phase 2 runs the receivers and the
@@ -308,27 +310,32 @@ int64_t edge_b200_last_launches(const edge_b200_ctx *ctx);
  * 2 = sources, 3 = receivers, the summed milliseconds and launch counts since timing was enabled
  * (synchronises the stream). */
 int edge_b200_set_timing(edge_b200_ctx *ctx, int enable);
-/* Fused GTS steps (1, the default; 0 turns them off): in configurations that pre-mix their face
- * projections and without halo parts, edge_b200_step with n_steps > 1 runs each step's neighbour
- * step inside the next step's local kernel (which adds the previous projections' lifted fluxes to
- * each element's DOF rows before its recursion; the receiver kernel does the same for its
- * elements), with the face projections alternating between two buffers; the last step's
- * neighbour step runs on its own before the call returns, so the DOFs are complete between calls.
- * Same arithmetic as the separate neighbour kernel: the results are identical. No counterpart in
- * the reference. */
+/* Fused GTS steps (1, the default; 0 turns them off): in the strong-form step and without halo
+ * parts, edge_b200_step with n_steps > 1 runs each step's surface integrals (own and neighbour
+ * flux, which arrive as three characteristic rows per face from each side) inside the next step's
+ * kernel, before its recursion; the receiver kernel does the same for its elements. The last step's
+ * surface integrals run on their own before the call returns, so the DOFs are complete between
+ * calls. Same arithmetic as the separate kernels: the results are identical. No counterpart in the
+ * reference.
+ * The strong form is taken by every configuration whose rows fit the kernels (all elastic ones; with
+ * 3 mechanisms up to order 5 in FP32 and order 4 in FP64) as long as every face's flux solvers, with
+ * the element's own flux across the face taken off, act through three waves -- Godunov fluxes of
+ * elastic media do; the first GTS step after the mesh or element data changed checks it. Otherwise
+ * GTS steps run the weak-form kernels, unfused. */
 int edge_b200_set_fused(edge_b200_ctx *ctx, int enable);
 int edge_b200_kernel_times(edge_b200_ctx *ctx, double *ms, int64_t *launches);
 /* Launch shape of the context's compiled configuration (no counterpart in the reference, whose
- * kernels run one element per thread team): info[0] elements per CTA, info[1] 1 when GTS face
- * projections leave the local kernel pre-mixed with the reading element's flux solver (the local
- * kernel then reads per element face the padded pair [2][info[2]] of flux solvers in the
- * configuration's precision, the neighbour kernel none), 2 when the local kernel does both of those
- * mixes through the rank-3 factors of the face's flux-solver pair (it then reads 108 factor values
- * per face instead of the pair; the form of the next GTS step once its factors are built),
- * info[3] / info[4] persistent CTAs of the
- * local / neighbour kernel, info[5] 1 when multi-step calls fuse each neighbour step into the next
- * local kernel (edge_b200_set_fused). */
+ * kernels run one element per thread team): info[0] elements per CTA, info[3] / info[4] persistent
+ * CTAs of the weak-form local / neighbour kernel. info[1], info[2] and info[5] describe the weak-form
+ * kernels' buffers: info[1] 1 when face projections leave the local kernel pre-mixed with the reading
+ * element's flux solver (per element face the padded pair [2][info[2]] of flux solvers in the
+ * configuration's precision), 2 when there is also room for the characteristic rows through which
+ * the LTS kernels mix, info[5] 1 when info[1] > 0 and fused steps are on. edge_b200_step_form tells
+ * which form the GTS steps take. */
 int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]);
+/* The form of the context's next GTS step (EDGE_B200_EINVAL before mesh and element data are set):
+ * 1 strong, 0 weak (see edge_b200_set_fused). Builds the step's coefficients if they are not built. */
+int edge_b200_step_form(edge_b200_ctx *ctx);
 
 /* No counterpart in the reference. n_steps GTS steps (local kernel, then neighbour kernel; no
  * sources, no receivers) over caller-owned DEVICE arrays, without allocating anything: no

@@ -1,0 +1,73 @@
+"""The strong-form GTS step is the one that runs: Godunov flux solvers of elastic and anelastic media
+are found to be of rank 3 (free surface, outflow, layered and jittered inner faces), other flux solvers
+send the context to the weak-form kernels, and both agree with the oracle."""
+import numpy as np
+import pytest
+
+from edge_b200._lib import lib
+from edge_b200.solver import Solver
+from helpers import OracleRun, random_dofs, rel_l2, small_problem
+
+pytestmark = pytest.mark.gpu
+
+# (order, runs, mechanisms, precision): every order, run count and both kinds of rows, odd group tails
+FORMS = [(2, 1, 0, 32), (2, 1, 0, 64), (3, 4, 0, 32), (4, 8, 0, 32), (5, 16, 0, 32), (5, 1, 0, 64), (6, 4, 0, 32),
+         (6, 1, 0, 64), (3, 16, 3, 32), (4, 8, 3, 32), (4, 1, 3, 64), (5, 4, 3, 32)]
+
+
+@pytest.mark.parametrize("order,runs,rm,prec", FORMS)
+def test_strong_form_runs_and_matches(order, runs, rm, prec):
+    prob = small_problem(n=(3, 2, 3), order=order, runs=runs, rm=rm, jitter=0.15, n_steps=6, source="random",
+                         layers=[3000.0, 6000.0], lognormal_sigma=0.2)
+    e0, a0 = random_dofs(prob, seed=4)
+    s = Solver(prob, precision=prec)
+    assert lib().edge_b200_step_form(s._h) == 1
+    s.upload_dofs(e0, a0)
+    for k in (1, 4):
+        s.step(k)
+    orc = OracleRun(prob, e0, a0)
+    orc.step(5)
+    e, a = s.download_dofs()
+    tol = 1e-12 if prec == 64 else 1e-4
+    assert rel_l2(e, orc.state["dofsE"]) < tol
+    if rm:
+        assert rel_l2(a, orc.state["dofsA"]) < tol
+    rb, _, rc = s.receivers()
+    k = int(rc[0])
+    assert k > 0 and rel_l2(rb[:, :k], orc.recv["buf"][:, :k]) < tol
+    s.close()
+
+
+def test_anelastic_order_6_keeps_the_weak_form():
+    prob = small_problem(n=2, order=6, runs=4, rm=3, n_steps=1, source=None, n_receivers=0)
+    s = Solver(prob, precision=32)
+    assert lib().edge_b200_step_form(s._h) == 0
+    s.close()
+
+
+@pytest.mark.parametrize("order,runs,rm,prec", [(4, 1, 0, 64), (5, 16, 0, 32), (4, 8, 3, 32)])
+def test_full_rank_flux_solvers_take_the_weak_form(order, runs, rm, prec):
+    """A penalty on the jump makes one inner face's flux solvers full rank: weak form, same results as
+    the oracle with those solvers; the next element data decide anew."""
+    prob = small_problem(n=2, order=order, runs=runs, rm=rm, jitter=0.1, n_steps=3, source=None, n_receivers=0)
+    good = prob.fsE.copy()
+    e, f = map(int, np.argwhere(prob.mesh.el_fa_type == 0)[5])
+    pen = 0.05 * np.abs(prob.fsE[0, e, f].reshape(9, 9)).max(axis=1).min() * np.eye(9)
+    prob.fsE[0, e, f] -= pen.ravel()
+    prob.fsE[1, e, f] += pen.ravel()
+    e0, a0 = random_dofs(prob, seed=8)
+    s = Solver(prob, precision=prec)
+    assert lib().edge_b200_step_form(s._h) == 0
+    s.upload_dofs(e0, a0)
+    s.step(3)
+    orc = OracleRun(prob, e0, a0)
+    orc.step(3)
+    got, _ = s.download_dofs()
+    assert rel_l2(got, orc.state["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
+    prob.fsE[:] = good
+    arr = [None if v is None else np.ascontiguousarray(v, np.float64)
+           for v in (prob.starE, prob.fsE, prob.starA, prob.srcA, prob.fsA, prob.omega)]
+    ptrs = [None if v is None else v.ctypes.data for v in arr]
+    assert lib().edge_b200_upload_element_data(s._h, *ptrs) == 0
+    assert lib().edge_b200_step_form(s._h) == 1
+    s.close()
