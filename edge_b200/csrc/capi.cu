@@ -278,6 +278,26 @@ __global__ void kSetRun(T *rows, const T *src, int64_t nRows, int B, int R, int 
 }
 }  // namespace
 
+// integrals of nSrc sources' series over nSteps steps of dt from s.t on (or of their own clocks):
+// out[step][source]. One thread per pair, so that the steps' source kernels, one after another on the
+// stream, only add (a series integral is a chain of FP64 divisions and loads, 8 of the 11 us that
+// kSources takes with it on a small mesh).
+static __global__ void kSrcIntegrals(SrcArgs s, int nSrc, int nSteps, double *out) {
+  const int64_t n = int64_t(nSrc) * nSteps;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const int k = int(i / nSrc), j = int(i % nSrc);
+    double a1 = s.t, a2;
+    if (s.clk0) {
+      a1 = s.clk0[j] + double(s.step + k) * s.clkDt[j];
+      a2 = a1 + s.clkDt[j];
+    } else {
+      for (int c = 0; c < k; c++) a1 += s.dt;  // the steps' times as the step loop forms them
+      a2 = a1 + s.dt;
+    }
+    out[i] = seriesIntegral(s.dts[j], s.t0[j], s.nPts[j], s.ts + s.tsOff[j], a1, a2, s.tol);
+  }
+}
+
 struct edge_b200_ctx {
   edge_b200_cfg cfg{};
   int64_t nEl = 0;
@@ -324,6 +344,7 @@ struct edge_b200_ctx {
   // sources
   SrcArgs src{};
   DevBuf srcMem[10];
+  DevBuf srcAmp;  // series integrals of the next steps (kSrcIntegrals)
   // per-source clocks and per-group time steps of merged simulations (edge_b200_set_source_clocks,
   // edge_b200_set_group_dt); srcStep counts the steps since the clocks were set
   DevBuf srcClk0, srcClkDt, grpDt;
@@ -1126,6 +1147,13 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
               "receiver schedule");
   }
   ctx->launches = 0;
+  // steps whose series integrals are computed together (one launch more, so not for a step or two),
+  // up to 1 MB of them at a time
+  int srcAhead = 1;
+  if (ctx->src.nGrp > 0 && ctx->rangeSrc && (phases & 1) && n_steps > 2) {
+    srcAhead = (int)std::min<int64_t>({int64_t(n_steps), 1024, std::max<int64_t>(1, 131072 / ctx->nSrc)});
+    EDGE_CUDA(ctx->srcAmp.fit(size_t(srcAhead) * ctx->nSrc * sizeof(double)), "source integrals");
+  }
   StepArgsRaw a = ctx->args(dt);
   if (ctx->rangeCount >= 0) {
     a.elFirst = ctx->rangeFirst;
@@ -1166,6 +1194,17 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
           sa.step = ctx->srcStep;
         }
         sa.dt = dt;
+        if (srcAhead > 1) {
+          if (st % srcAhead == 0) {
+            const int nAhead = std::min(srcAhead, n_steps - st);
+            const int64_t n = int64_t(ctx->nSrc) * nAhead;
+            kSrcIntegrals<<<(int)std::min<int64_t>((n + 63) / 64, 148 * 8), 64, 0, s>>>(sa, ctx->nSrc, nAhead,
+                                                                                      ctx->srcAmp.as<double>());
+            EDGE_CUDA(cudaGetLastError(), "source integrals");
+            ctx->launches++;
+          }
+          sa.amp = ctx->srcAmp.as<double>() + size_t(st % srcAhead) * ctx->nSrc;
+        }
         EDGE_CUDA(ctx->launch(2, [&] { return ctx->ks->sources(ctx->dofsE, sa, s); }), "source kernel");
         ctx->launches++;
       }
