@@ -183,20 +183,30 @@ __global__ void kBuildFsChar(const double *fsE, const int32_t *elFaEl, const uin
   }
 }
 
-// halo exchange: blocks of blk16 x 16 bytes of face slots (element * 4 + face) to / from a packed
-// buffer with stride16 x 16 bytes per slot, 16 bytes per thread; slots outside the face buffer are
-// skipped
-__global__ void kFacePack(uint4 *face, uint4 *buf, const int32_t *slots, int n, int64_t blk16, int64_t stride16,
-                          int64_t nSlots, bool pack) {
-  const int64_t total = (int64_t)n * blk16;
+// halo exchange: the rows of face slots (element * 4 + face) to / from a packed buffer with stride16 x
+// 16 bytes per slot, 16 bytes per thread; slots outside the face buffer are skipped. Weak form: nine
+// pre-mixed rows; strong form: three characteristic rows and a mark behind them, by which a part
+// notices rows of the other form (*bad counts them; they are not taken over).
+constexpr uint4 kHaloMark = {0x7fa5c3e1u, 0x51e0c4a7u, 0x7fe1a5c3u, 0x0c4a751eu};
+__global__ void kFacePack(uint4 *face, uint4 *buf, const int32_t *slots, int n, int64_t stride16, int64_t nSlots,
+                          bool strong, bool pack, int *bad) {
+  const int64_t blk16 = strong ? stride16 / 3 : stride16, total = (int64_t)n * blk16;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t k = i / blk16, w = i % blk16;
     const int64_t sl = slots[k];
     if (sl < 0 || sl >= nSlots) continue;
-    if (pack)
+    uint4 *mark = buf + k * stride16 + stride16 / 3;
+    if (pack) {
       buf[k * stride16 + w] = face[sl * blk16 + w];
-    else
+      if (strong && w == 0) *mark = kHaloMark;
+      continue;
+    }
+    const uint4 m = *mark;
+    const bool isStrong = m.x == kHaloMark.x && m.y == kHaloMark.y && m.z == kHaloMark.z && m.w == kHaloMark.w;
+    if (isStrong == strong)
       face[sl * blk16 + w] = buf[k * stride16 + w];
+    else if (w == 0)
+      atomicAdd(bad, 1);
   }
 }
 
@@ -341,6 +351,7 @@ struct edge_b200_ctx {
   bool pending = false, fusedOn = true;
   char *faceThird(int i) const { return static_cast<char *>(face) + i * (faceCount() / 3 * realSize); }
   void *outBuf(int i) const { return faceThird(i); }
+  DevBuf haloBad;  // blocks unpacked in the other form (kFacePack)
   // sources
   SrcArgs src{};
   DevBuf srcMem[10];
@@ -633,6 +644,17 @@ struct edge_b200_ctx {
     charRejected = stepRejected = false;
   }
 
+  // after the stream was waited for: whether a part's rows arrived in the other form
+  int checkHalo() {
+    if (!haloBad.p) return EDGE_B200_OK;
+    int n = 0;
+    cudaError_t e = cudaMemcpy(&n, haloBad.p, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e) return fail(e, "halo check");
+    if (n == 0) return EDGE_B200_OK;
+    err = "halo rows of the other step form arrived: the flux solvers of only some parts have rank 3";
+    return EDGE_B200_EMESH;
+  }
+
   int fail(cudaError_t e, const char *what) {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return EDGE_B200_EDEVICE;
@@ -848,7 +870,7 @@ int edge_b200_download_dofs(edge_b200_ctx *ctx, void *dofs_e, void *dofs_a) {
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
   EDGE_CUDA(ctx->downloadRows(dofs_e, ctx->dofsE, 9), "download dofsE");
   if (ctx->cfg.n_rms && dofs_a) EDGE_CUDA(ctx->downloadRows(dofs_a, ctx->dofsA, 6 * ctx->cfg.n_rms), "download dofsA");
-  return EDGE_B200_OK;
+  return ctx->checkHalo();
 }
 
 int edge_b200_upload_dofs_async(edge_b200_ctx *ctx, const void *dofs_e, const void *dofs_a) {
@@ -1274,13 +1296,17 @@ static int packFaces(edge_b200_ctx *ctx, int n, const int32_t *slots, void *buf,
   if (!ctx || n < 0 || (n && (!slots || !buf))) return EDGE_B200_EINVAL;
   if (n == 0) return EDGE_B200_OK;
   if (ctx->meshSet && ctx->dataSet) EDGE_CUDA(ctx->ensureGts(), "step coefficients");
-  // strong form: the three characteristic rows of the slot, at the start of its block
+  if (!ctx->haloBad.p) {
+    EDGE_CUDA(ctx->haloBad.fit(sizeof(int)), "halo check");
+    EDGE_CUDA(cudaMemsetAsync(ctx->haloBad.p, 0, sizeof(int), ctx->stream), "halo check");
+  }
   const bool st = ctx->strong();
-  const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16, blk16 = st ? stride16 / 3 : stride16;
-  const int64_t total = (int64_t)n * blk16;
+  const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16;
+  const int64_t total = (int64_t)n * (st ? stride16 / 3 : stride16);
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
   kFacePack<<<grid, 256, 0, ctx->stream>>>(static_cast<uint4 *>(st ? ctx->outBuf(ctx->outCur) : ctx->face),
-                                           static_cast<uint4 *>(buf), slots, n, blk16, stride16, ctx->nEl * 4, pack);
+                                           static_cast<uint4 *>(buf), slots, n, stride16, ctx->nEl * 4, st, pack,
+                                           ctx->haloBad.as<int>());
   EDGE_CUDA(cudaGetLastError(), pack ? "pack faces" : "unpack faces");
   return EDGE_B200_OK;
 }
@@ -1591,7 +1617,7 @@ int edge_b200_sync(edge_b200_ctx *ctx) {
   if (ctx->h2d) EDGE_CUDA(cudaStreamSynchronize(ctx->h2d), "sync");
   if (ctx->d2h) EDGE_CUDA(cudaStreamSynchronize(ctx->d2h), "sync");
   EDGE_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-  return EDGE_B200_OK;
+  return ctx->checkHalo();
 }
 
 int edge_b200_device_dofs(edge_b200_ctx *ctx, void **dofs_e, void **dofs_a, void **tdofs) {
