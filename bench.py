@@ -143,37 +143,33 @@ def host_n_modes(order):
     return order * (order + 1) * (order + 2) // 6
 
 
-def algorithmic(prob, prec, premix=False, fs_pair=84, fused=False, char=False):
-    """Per-element algorithmic bytes and flops of one step (dense-in-modes counts as in the
-    roofline model of the path) for each kernel. premix: the local kernel mixes the face
-    projections with the reading element's flux solver and reads per face the padded pair
-    [2][fs_pair] of flux solvers in the compute precision instead of its own fsE[0] block; the
-    neighbour kernel then reads no flux solvers. char: the local kernel mixes through the rank-3
-    factors of each face's flux-solver pair (3 x 9 + 2 x 9 x 3 products per face mode for both
-    mixes instead of 2 x 81) and reads 108 factor values per face instead of the pair. fused: the
-    local kernel also runs the previous step's neighbour step (reads the four neighbour projections
-    and the connectivity, adds their lifted fluxes and stores the completed DOF rows once more)."""
+def algorithmic(prob, prec, strong):
+    """Per-element bytes and flops of one step (products counted dense in modes) of the two kernels.
+    strong: the step kernel runs a whole step per launch -- DOFs read and written, per face three
+    characteristic rows from each side read and written, the element's coefficients (U, star rows,
+    V) -- the neighbour kernel the closing surface integrals of a call. Otherwise the weak-form
+    kernels: nine face rows each way, FP64 star matrices and flux solvers."""
     from edge_b200.host import n_face_modes, n_modes
     O, R, rm = prob.order, prob.runs, prob.rm
     B, F, p = n_modes(O), n_face_modes(O), (8 if prec == 64 else 4)
     Bm = lambda o: n_modes(o) if o > 0 else 0
     ck = sum(3 * (2 * 9 * Bm(O - d) * Bm(O - d + 1) + 2 * 24 * Bm(O - d)) + 2 * 9 * Bm(O - d) for d in range(1, O))
+    dofs = (9 + 6 * rm) * B * R * p
+    if strong:
+        nq = 15 if rm else 9
+        rows = 4 * 3 * F * R * p
+        lift_bytes = 2 * dofs + 2 * rows + 4 * nq * 3 * p + 16
+        lift_flops = 4 * (2 * nq * 3 * F + 2 * nq * F * B) * R
+        coef = (4 * nq * 3 + 81 + 4 * 9 * 6 + ((36 + 12 * rm) if rm else 0)) * p + 16
+        return dict(local_bytes=2 * dofs + 4 * rows + coef, neigh_bytes=lift_bytes, neigh_flops=lift_flops,
+                    local_flops=(ck + 4 * (2 * 9 * F * B + 2 * 9 * 6 * F)) * R + lift_flops)
     vol = 3 * (2 * 9 * B * Bm(O - 1) + 2 * 24 * B)
     surf = 4 * (2 * 9 * F * B + 2 * 81 * F + 2 * 9 * B * F)
-    dofs = (9 + 6 * rm) * B * R * p
     face = 4 * 9 * F * R * p
-    fs_local = 4 * 108 * p if char else (4 * 2 * fs_pair * p if premix else 4 * 81 * 8)
-    local_bytes = 2 * dofs + face + 3 * 24 * 8 + fs_local + (rm * 12 * 8 + 27 * 8 + 4 * 54 * 8 if rm else 0)
-    neigh_bytes = 2 * dofs + face + (0 if premix else 4 * 81 * 8) + 4 * (4 + 1 + 1 + 1) + (4 * 54 * 8 if rm else 0)
-    # the face mixes: surf counts one 9 x 9 mix per face; pre-mixing adds the second, and the
-    # factors replace both by 3 x 9 + 2 x 9 x 3 products per face mode
-    mix = (4 * 2 * (81 + 54 - 2 * 81) * F if char else 0) + (4 * 2 * 81 * F if premix else 0)
-    local_flops = (ck + vol + surf + mix) * R
-    neigh_flops = (surf - 4 * 2 * 81 * F) * R if premix else surf * R
-    if fused:
-        local_bytes += face + dofs + 4 * (4 + 1 + 1 + 1)
-        local_flops += neigh_flops
-    return dict(local_bytes=local_bytes, neigh_bytes=neigh_bytes, local_flops=local_flops, neigh_flops=neigh_flops)
+    local_bytes = 2 * dofs + face + 3 * 24 * 8 + 4 * 81 * 8 + (rm * 12 * 8 + 27 * 8 + 4 * 54 * 8 if rm else 0)
+    neigh_bytes = 2 * dofs + face + 4 * 81 * 8 + 4 * (4 + 1 + 1 + 1) + (4 * 54 * 8 if rm else 0)
+    return dict(local_bytes=local_bytes, neigh_bytes=neigh_bytes, local_flops=(ck + vol + surf) * R,
+                neigh_flops=surf * R)
 
 
 def compulsory_step_bytes(prob, prec):
@@ -209,7 +205,7 @@ def peak_clock_mhz():
 
 def traffic_from_profiles(workload):
     """Per-launch DRAM bytes of the dominant kernel from the committed ncu summary, if present."""
-    path = os.path.join(ROOT, "profiles", f"kLocal_{workload}.txt")
+    path = os.path.join(ROOT, "profiles", f"kStep_{workload}.txt")
     try:
         for line in open(path):
             if line.startswith("dram_bytes_per_full_launch:"):
@@ -843,17 +839,16 @@ def main():
     L.edge_b200_set_timing(sv._h, 0)
     names = ["local", "neighbour", "sources", "receivers"]
     shares = {names[i]: float(kms[i] / kms.sum()) for i in range(4) if kn[i]}
-    kc = np.zeros(6, np.int32)
-    L.edge_b200_kernel_config(sv._h, _lib.ptr(kc))
-    alg = algorithmic(prob, prec, premix=bool(kc[1]), fs_pair=int(kc[2]), fused=bool(kc[5]), char=int(kc[1]) == 2)
+    strong = L.edge_b200_step_form(sv._h) == 1
+    alg = algorithmic(prob, prec, strong)
     top = int(np.argmax(kms[:2]))
     avg_ms = kms[top] / max(kn[top], 1)
     # algorithmic bytes: the path's compulsory bytes of one element step (every array touched once:
     # DOFs read + written, time-integrated DOFs written + read once, FP64 star matrices and flux
-    # solvers, connectivity) times the elements of the launch. The fused local kernel runs a whole
-    # step per launch (this step's local update and the previous step's neighbour update); without
-    # fusion the step's two kernels are timed together.
-    fused = bool(kc[5])
+    # solvers, connectivity) times the elements of the launch. The strong-form step kernel runs a
+    # whole step per launch (the previous step's surface integrals and this step's update up to its
+    # own); the weak-form step's two kernels are timed together.
+    fused = strong
     step_bytes = compulsory_step_bytes(prob, prec)
     bytes_launch = step_bytes * prob.n_el
     launch_ms = avg_ms if (fused and top == 0) else (kms[0] / max(kn[0], 1) + kms[1] / max(kn[1], 1))
@@ -881,9 +876,9 @@ def main():
         roofline["fp32_pipe"] = {"dense_equivalent_tflops": roofline["achieved_tflops"],
                                  "nominal_peak_tflops": fp32_peak,
                                  "frac": roofline["achieved_tflops"] / fp32_peak}
-    # the neighbour-flux kernel (the HBM-bound one) on its own: bytes this design moves (face
-    # projections read, DOFs read + written, flux solvers, connectivity) and the reference algorithm's
-    # count (neighbours' time-integrated DOFs instead of face projections)
+    # the neighbour-flux kernel (the HBM-bound one) on its own: bytes this design moves (DOFs read +
+    # written, face rows, coefficients) and the reference algorithm's count (neighbours'
+    # time-integrated DOFs instead of face rows)
     n_ms = kms[1] / max(kn[1], 1)
     B_, F_, p_ = host_n_modes(prob.order), prob.order * (prob.order + 1) // 2, (8 if prec == 64 else 4)
     ref_bytes = (3 * 9 * B_ * prob.runs * p_ + 4 * 81 * 8 + 4 * 6) * prob.n_el

@@ -96,93 +96,6 @@ __global__ void kBuildFsLR(const double *fsE, const int32_t *elFaEl, const uint8
   }
 }
 
-// characteristic factors of the same pairs (Geo::charMix): per element face the stacked flux
-// solvers S = [fsE[0]; the reader's fsE[1]] (18 x 9, zeros for an outflow reader) have rank 3 --
-// the waves leaving the element through the face -- so S = U V^T with U 18 x 3 and V 9 x 3. The
-// columns of S (inputs: stresses and velocities, whose scales differ by the impedances) are
-// scaled to unit maximum, c; Gram-Schmidt with pivoting over the 18 scaled rows (each new
-// direction orthogonalised twice) gives Q (3 orthonormal directions); then U = (S / c) Q^T and
-// V = c Q. out[nEl][4][2][P]: V [9][4] (column 3 zero), then per quantity q {U0[q][0..2],
-// U1[q][0..2], 0, 0}, the rest zero; a face whose scaled rows keep more than 1e-9 of the largest
-// row's norm outside the three directions counts in *bad (its pair is not of rank 3).
-template <typename T>
-__global__ void kBuildFsChar(const double *fsE, const int32_t *elFaEl, const uint8_t *fId, const uint8_t *faType,
-                             int64_t nEl, int P, T *out, int *bad) {
-  for (int64_t ef = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; ef < nEl * 4;
-       ef += int64_t(gridDim.x) * blockDim.x) {
-    const double *A = fsE + ef * 81;
-    const double *Bm = nullptr;
-    const int ty = faType[ef];
-    if (ty == EDGE_FACE_INNER)
-      Bm = fsE + ((nEl + elFaEl[ef]) * 4 + fId[ef]) * 81;
-    else if (ty == EDGE_FACE_FREE_SURFACE)
-      Bm = fsE + (nEl * 4 + ef) * 81;
-    auto entry = [&](int i, int j) { return i < 9 ? A[i * 9 + j] : (Bm ? Bm[(i - 9) * 9 + j] : 0.0); };
-    double c[9];
-    for (int j = 0; j < 9; j++) {
-      double m = 0;
-      for (int i = 0; i < 18; i++) m = fmax(m, fabs(entry(i, j)));
-      c[j] = m > 0 ? m : 1.0;
-    }
-    double rs[18][9], nrm0 = 0;
-    for (int i = 0; i < 18; i++) {
-      double n2 = 0;
-      for (int j = 0; j < 9; j++) {
-        rs[i][j] = entry(i, j) / c[j];
-        n2 += rs[i][j] * rs[i][j];
-      }
-      nrm0 = fmax(nrm0, n2);
-    }
-    double Q[3][9];
-    for (int k = 0; k < 3; k++) {
-      int piv = 0;
-      double best = -1;
-      for (int i = 0; i < 18; i++) {
-        double n2 = 0;
-        for (int j = 0; j < 9; j++) n2 += rs[i][j] * rs[i][j];
-        if (n2 > best) {
-          best = n2;
-          piv = i;
-        }
-      }
-      double v[9];
-      for (int j = 0; j < 9; j++) v[j] = rs[piv][j];
-      for (int pass = 0; pass < 2; pass++)
-        for (int kk = 0; kk < k; kk++) {
-          double d = 0;
-          for (int j = 0; j < 9; j++) d += v[j] * Q[kk][j];
-          for (int j = 0; j < 9; j++) v[j] -= d * Q[kk][j];
-        }
-      double n2 = 0;
-      for (int j = 0; j < 9; j++) n2 += v[j] * v[j];
-      const double inv = n2 > 1e-60 * nrm0 && n2 > 0 ? 1.0 / sqrt(n2) : 0.0;
-      for (int j = 0; j < 9; j++) Q[k][j] = v[j] * inv;
-      for (int i = 0; i < 18; i++) {
-        double d = 0;
-        for (int j = 0; j < 9; j++) d += rs[i][j] * Q[k][j];
-        for (int j = 0; j < 9; j++) rs[i][j] -= d * Q[k][j];
-      }
-    }
-    double res = 0;
-    for (int i = 0; i < 18; i++) {
-      double n2 = 0;
-      for (int j = 0; j < 9; j++) n2 += rs[i][j] * rs[i][j];
-      res = fmax(res, n2);
-    }
-    if (res > 1e-18 * nrm0) atomicAdd(bad, 1);
-    T *o = out + ef * 2 * P;
-    for (int j = 0; j < 2 * P; j++) o[j] = T(0);
-    for (int j = 0; j < 9; j++)
-      for (int k = 0; k < 3; k++) o[4 * j + k] = T(c[j] * Q[k][j]);
-    for (int i = 0; i < 18; i++)
-      for (int k = 0; k < 3; k++) {
-        double u = 0;
-        for (int j = 0; j < 9; j++) u += entry(i, j) / c[j] * Q[k][j];
-        o[36 + (i % 9) * 8 + (i / 9) * 3 + k] = T(u);
-      }
-  }
-}
-
 // halo exchange: the rows of face slots (element * 4 + face) to / from a packed buffer with stride16 x
 // 16 bytes per slot, 16 bytes per thread; slots outside the face buffer are skipped. Weak form: nine
 // pre-mixed rows; strong form: three characteristic rows and a mark behind them, by which a part
@@ -333,13 +246,12 @@ struct edge_b200_ctx {
   // rebuilt before the next GTS step after the mesh or the element data changed
   DevBuf fsLR;
   bool fsLRStale = true;
-  bool fsLRChar = false;      // fsLR holds the characteristic factors of the pairs
-  DevBuf charBad;             // device counter of the factor build's rank check
-  bool charRejected = false;  // some face's pair is not of rank 3 (until the element data changes)
   // strong-form GTS steps (step.cuh): coefficients and gather table, rebuilt before the next GTS step
   // after the mesh or the element data changed; flux solvers that are not of rank 3 in that form
   // keep the context on the weak-form kernels until the data change again
-  DevBuf fac, gath, stepBad;
+  void *fac = nullptr;  // fac, gath and stepBad lie behind the face buffer, in its allocation
+  uint32_t *gath = nullptr;
+  int *stepBad = nullptr;
   bool stepStale = true, stepRejected = false;
   bool strong() const { return ks->strongSupported() && !stepStale && !stepRejected; }
   // the face buffer ([nEl][4][9][R][GF]) then holds the characteristics the elements write for their
@@ -447,6 +359,22 @@ struct edge_b200_ctx {
   size_t faceCount() const { return (size_t)nEl * 4 * 9 * cfg.n_runs * GF; }
   // the last third of the face buffer takes the own characteristics of whole element groups (32 lanes)
   size_t faceAlloc() const { return faceCount() + (size_t)32 * 12 * GF; }
+  // face buffer and, for configurations with the strong-form step, its coefficients (whole groups of E
+  // elements) and gather table: one allocation, none left for the first step
+  cudaError_t allocFace() {
+    const auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t E = ks->elementsPerCta(), len = cfg.n_rms ? FacL<3>::src + 12 * cfg.n_rms + 288 : FacL<0>::len;
+    const size_t bFace = up(faceAlloc() * realSize), bFac = up((nEl + E - 1) / E * E * len * realSize);
+    const size_t bGath = up(size_t(nEl) * 4 * sizeof(uint32_t));
+    const bool strongToo = ks->strongSupported();
+    cudaError_t e = cudaMalloc(&face, bFace + (strongToo ? bFac + bGath + 256 : 0));
+    if (e || !strongToo) return e;
+    char *p = static_cast<char *>(face) + bFace;
+    fac = p;
+    gath = reinterpret_cast<uint32_t *>(p + bFac);
+    stepBad = reinterpret_cast<int *>(p + bFac + bGath);
+    return cudaSuccess;
+  }
   size_t refCount(int rows) const { return (size_t)nEl * rows * B * cfg.n_runs; }
   cudaError_t ensureStage() {
     if (stage) return cudaSuccess;
@@ -554,42 +482,12 @@ struct edge_b200_ctx {
     return cudaSuccess;
   }
 
-  // the flux-solver pairs of the pre-mixed projections (weak form): as characteristic factors for the
-  // LTS steps of a configuration whose kernels mix through them (unless some face's pair is not of
-  // rank 3, found when the factors are built: the pairs themselves from then on until the element
-  // data changes), else as the pairs themselves
-  cudaError_t ensureFsLR(bool lts = false) {
-    if (!ks->premix()) return cudaSuccess;
-    const bool wantChar = lts && ks->charMixLts() && !charRejected;
-    if (!fsLRStale && fsLRChar == wantChar) return cudaSuccess;
+  // the flux-solver pairs of the pre-mixed projections (weak form)
+  cudaError_t ensureFsLR() {
+    if (!ks->premix() || !fsLRStale) return cudaSuccess;
     const int P = ks->fsPairStride();
     cudaError_t e = fsLR.fit(size_t(nEl) * 4 * 2 * P * realSize);
     if (e) return e;
-    if (wantChar) {
-      // the count of faces whose pair is not of rank 3, read back once (no allocation or device-wide
-      // synchronisation on the way: pools of a server set themselves up while others run)
-      if ((e = charBad.fit(sizeof(int)))) return e;
-      int *bad = charBad.as<int>();
-      int nBad = 0;
-      e = cudaMemsetAsync(bad, 0, sizeof(int), stream);
-      if (!e) {
-        const int grid = (int)std::min<int64_t>((nEl * 4 + 127) / 128, 148 * 8);
-        if (cfg.precision == 64)
-          kBuildFsChar<double><<<grid, 128, 0, stream>>>(fsE, elFaEl, fId, faType, nEl, P, fsLR.as<double>(), bad);
-        else
-          kBuildFsChar<float><<<grid, 128, 0, stream>>>(fsE, elFaEl, fId, faType, nEl, P, fsLR.as<float>(), bad);
-        e = cudaGetLastError();
-      }
-      if (!e) e = cudaMemcpyAsync(&nBad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream);
-      if (!e) e = cudaStreamSynchronize(stream);
-      if (e) return e;
-      if (nBad == 0) {
-        fsLRStale = false;
-        fsLRChar = true;
-        return cudaSuccess;
-      }
-      charRejected = true;
-    }
     const int64_t total = nEl * 4 * 2 * P;
     const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
     if (cfg.precision == 64)
@@ -598,7 +496,6 @@ struct edge_b200_ctx {
       kBuildFsLR<float><<<grid, 256, 0, stream>>>(fsE, elFaEl, fId, faType, nEl, P, fsLR.as<float>());
     if ((e = cudaGetLastError())) return e;
     fsLRStale = false;
-    fsLRChar = false;
     return cudaSuccess;
   }
 
@@ -610,23 +507,19 @@ struct edge_b200_ctx {
       return cudaSuccess;
     }
     cudaError_t e;
-    const int len = cfg.n_rms ? FacL<3>::src + 12 * cfg.n_rms + 288 : FacL<0>::len;
-    const int E = ks->elementsPerCta();  // the layout's interleaving: whole groups of E elements
-    if ((e = fac.fit(size_t((nEl + E - 1) / E * E) * len * realSize)) || (e = gath.fit(size_t(nEl) * 4 * sizeof(uint32_t))) ||
-        (e = stepBad.fit(sizeof(int))))
-      return e;
+    const int E = ks->elementsPerCta();
     // the count of faces not of rank 3 is read back once (no allocation of its own or device-wide
     // synchronisation on the way: pools of a server set themselves up while others run)
-    int *bad = stepBad.as<int>(), nBad = 0;
+    int *bad = stepBad, nBad = 0;
     if ((e = cudaMemsetAsync(bad, 0, sizeof(int), stream))) return e;
-    const int64_t work = (nEl * 8 + kTeams * kBuildWarps - 1) / (kTeams * kBuildWarps);
+    const int64_t work = (nEl * 4 + kTeams * kBuildWarps - 1) / (kTeams * kBuildWarps);
     const int grid = (int)std::min<int64_t>(work, 148 * 32);
     if (cfg.precision == 64)
       kBuildStep<double><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
-                                                  fac.as<double>(), gath.as<uint32_t>(), bad);
+                                                  static_cast<double *>(fac), gath, bad);
     else
       kBuildStep<float><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
-                                                 fac.as<float>(), gath.as<uint32_t>(), bad);
+                                                 static_cast<float *>(fac), gath, bad);
     if ((e = cudaGetLastError())) return e;
     if ((e = cudaMemcpyAsync(&nBad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream))) return e;
     if ((e = cudaStreamSynchronize(stream))) return e;
@@ -641,7 +534,7 @@ struct edge_b200_ctx {
   }
   void dataChanged() {
     fsLRStale = stepStale = true;
-    charRejected = stepRejected = false;
+    stepRejected = false;
   }
 
   // after the stream was waited for: whether a part's rows arrived in the other form
@@ -666,8 +559,8 @@ struct edge_b200_ctx {
     a.dofsA = dofsA;
     a.tDofs = keepTDofs ? tDofs : nullptr;
     if (strong() && !weak) {
-      a.fac = fac.p;
-      a.gath = gath.as<uint32_t>();
+      a.fac = fac;
+      a.gath = gath;
       a.face = outBuf(outCur);
       a.wOwn = faceThird(2);
     } else {
@@ -683,7 +576,6 @@ struct edge_b200_ctx {
     a.vId = vId;
     a.faType = faType;
     a.fsLR = (ks->premix() && !fsLRStale) ? fsLR.p : nullptr;
-    a.fsChar = (a.fsLR && fsLRChar) ? 1 : 0;
     a.grpDt = grpDtOn ? grpDt.as<double>() : nullptr;
     a.nEl = nEl;
     a.elFirst = 0;
@@ -766,7 +658,7 @@ int edge_b200_create(const edge_b200_cfg *cfg, int64_t n_el, edge_b200_ctx **out
   size_t rs = ctx->realSize;
   if ((e = cudaMalloc(&ctx->dofsE, ctx->dofsCount() * rs)) ||
       (cfg->n_rms && (e = cudaMalloc(&ctx->dofsA, ctx->dofsACount() * rs))) ||
-      (e = cudaMalloc(&ctx->face, ctx->faceAlloc() * rs))) {
+      (e = ctx->allocFace())) {
     delete ctx;
     return e == cudaErrorMemoryAllocation ? EDGE_B200_ENOMEM : EDGE_B200_EDEVICE;
   }
@@ -1382,7 +1274,10 @@ int edge_b200_step_lts(edge_b200_ctx *ctx, double t, double dt_fun, int n_cycles
   if (!ctx->meshSet || !ctx->dataSet) return EDGE_B200_EINVAL;
   if (!ctx->ks->ltsSupported()) return EDGE_B200_ENOTSUP;
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
-  EDGE_CUDA(ctx->ensureFsLR(true), "flux-solver pairs");
+  // strong form as in GTS where the configuration's LTS kernels have it
+  if (ctx->ks->strongLts()) EDGE_CUDA(ctx->ensureStep(), "step coefficients");
+  const bool weak = !ctx->ks->strongLts() || !ctx->strong();
+  if (weak) EDGE_CUDA(ctx->ensureFsLR(), "flux-solver pairs");
   ctx->lastLts = true;
   const int G = ctx->nTg;
   const int64_t nFun = int64_t(1) << (G - 1);  // fundamental steps per cycle (largest group's step)
@@ -1448,7 +1343,7 @@ int edge_b200_step_lts(edge_b200_ctx *ctx, double t, double dt_fun, int n_cycles
   }
   ctx->launches = 0;
   for (const Work &w : work) {
-    StepArgsRaw a = ctx->args(w.dt, true);
+    StepArgsRaw a = ctx->args(w.dt, weak);
     a.elFirst = ctx->tgFirst[w.g];
     a.elCount = ctx->tgFirst[w.g + 1] - ctx->tgFirst[w.g];
     a.faceSum = ctx->faceSum.p;
@@ -1635,7 +1530,7 @@ int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]) {
   if (!ctx || !info) return EDGE_B200_EINVAL;
   info[5] = (ctx->fusedOn && ctx->ks->premix() && ctx->nOwned == ctx->nEl) ? 1 : 0;
   info[0] = ctx->ks->elementsPerCta();
-  info[1] = ctx->ks->premix() ? ((ctx->ks->charMix() && !ctx->charRejected) ? 2 : 1) : 0;
+  info[1] = ctx->ks->premix() ? (ctx->ks->strongSupported() && !ctx->stepRejected ? 2 : 1) : 0;
   info[2] = ctx->ks->fsPairStride();
   info[3] = ctx->ks->ctasLocal();
   info[4] = ctx->ks->ctasNeigh();

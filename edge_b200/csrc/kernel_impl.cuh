@@ -48,7 +48,6 @@ class KernelSetImpl final : public KernelSet {
     b.halfIdx = a.halfIdx;
     b.firstTs = a.firstTs;
     b.fsLR = static_cast<const T *>(a.fsLR);
-    b.fsChar = a.fsChar;
     b.fac = static_cast<const T *>(a.fac);
     b.gath = a.gath;
     b.wOwn = static_cast<T *>(a.wOwn);
@@ -92,6 +91,13 @@ class KernelSetImpl final : public KernelSet {
       if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occStep_, kStep<T, O, R>, S::NT, S::smem))) return e;
       if ((e = cudaFuncSetAttribute(kLift<T, O, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smemLift)))
         return e;
+      if constexpr (G::ltsOk) {
+        if ((e = cudaFuncSetAttribute(kStep<T, O, R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem)) ||
+            (e = cudaFuncSetAttribute(kStep<T, O, R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem)) ||
+            (e = cudaFuncSetAttribute(kLift<T, O, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)S::smemLift)))
+          return e;
+      }
       if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLift_, kLift<T, O, R>, S::NT, S::smemLift))) return e;
       occStep_ = occStep_ < 1 ? 1 : occStep_;
       occLift_ = occLift_ < 1 ? 1 : occLift_;
@@ -118,14 +124,6 @@ class KernelSetImpl final : public KernelSet {
                                                              G::smemLocalSums)))
         return e;
       occLocalSum_ = occLocalSum_ < 1 ? 1 : occLocalSum_;
-      if constexpr (G::charMixLts) {
-        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 2, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smemLocalLts)))
-          return e;
-        if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 1, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smemLocalSums)))
-          return e;
-      }
     }
     occLocal_ = occLocal_ < 1 ? 1 : occLocal_;
     occNeigh_ = occNeigh_ < 1 ? 1 : occNeigh_;
@@ -165,13 +163,14 @@ class KernelSetImpl final : public KernelSet {
     return cudaGetLastError();
   }
   bool strongSupported() const override { return RM == 0 || viscStrong; }
+  bool strongLts() const override { return RM == 0 && G::ltsOk; }
   cudaError_t localLts(const StepArgsRaw &a, cudaStream_t s) override {
     if constexpr (G::ltsOk) {
       if (a.elCount < 1) return cudaSuccess;
-      if constexpr (G::charMixLts) {
-        if (a.fsChar) {
-          kLocal<T, O, R, RM, 2, true>
-              <<<grid(a.elCount, numSms_ * occLocalLts_), G::NT, G::smemLocalLts, s>>>(cast(a));
+      if constexpr (RM == 0) {
+        using S = SGeo<T, O, R>;
+        if (a.fac) {
+          kStep<T, O, R, 2><<<grid(a.elCount, numSms_), S::NT, S::smem, s>>>(cast(a));
           return cudaGetLastError();
         }
       }
@@ -184,10 +183,10 @@ class KernelSetImpl final : public KernelSet {
   cudaError_t localLtsSums(const StepArgsRaw &a, cudaStream_t s) override {
     if constexpr (G::ltsOk) {
       if (a.elCount < 1) return cudaSuccess;
-      if constexpr (G::charMixLts) {
-        if (a.fsChar) {
-          kLocal<T, O, R, RM, 1, true>
-              <<<grid(a.elCount, numSms_ * occLocalSum_), G::NT, G::smemLocalSums, s>>>(cast(a));
+      if constexpr (RM == 0) {
+        using S = SGeo<T, O, R>;
+        if (a.fac) {
+          kStep<T, O, R, 1><<<grid(a.elCount, numSms_ * occStep_), S::NT, S::smem, s>>>(cast(a));
           return cudaGetLastError();
         }
       }
@@ -200,8 +199,6 @@ class KernelSetImpl final : public KernelSet {
   bool ltsSupported() const override { return G::ltsOk; }
   bool premix() const override { return G::premix; }
   int fsPairStride() const override { return G::FSP; }
-  bool charMix() const override { return G::charMix; }
-  bool charMixLts() const override { return G::charMixLts; }
   cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
     if constexpr (viscStrong) {
@@ -224,6 +221,13 @@ class KernelSetImpl final : public KernelSet {
   }
   cudaError_t neighLts(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;
+    if constexpr (RM == 0 && G::ltsOk) {
+      using S = SGeo<T, O, R>;
+      if (a.fac) {
+        kLift<T, O, R, true><<<grid(a.elCount, numSms_ * occLift_), S::NT, S::smemLift, s>>>(cast(a));
+        return cudaGetLastError();
+      }
+    }
     kNeigh<T, O, R, RM, G::premixLts><<<grid(a.elCount, ctasNeigh()), G::NT, smemNeigh(), s>>>(cast(a));
     return cudaGetLastError();
   }

@@ -25,10 +25,8 @@ struct StepArgsRaw {
   const int32_t *sumIdx = nullptr, *halfIdx = nullptr;
   int firstTs = 0;
   // per element face fsE[0] and the face reader's fsE[1] in the configuration's precision, each
-  // padded to 16 bytes: [nEl][4][2][fsPairStride()] (premix); fsChar: their characteristic
-  // factors instead (charMixLts)
+  // padded to 16 bytes: [nEl][4][2][fsPairStride()] (premix)
   const void *fsLR = nullptr;
-  int fsChar = 0;
   // strong-form GTS steps (StepArgs): coefficients (null: the weak-form kernels), gather table, own
   // characteristics, and the characteristics of the previous step that are still pending
   const void *fac = nullptr;
@@ -49,6 +47,8 @@ class KernelSet {
   // the configuration has the strong-form step (step.cuh), whose closing half neigh runs when a.fac
   // is given
   virtual bool strongSupported() const = 0;
+  // its LTS kernels too (localLts, localLtsSums and neighLts when a.fac is given)
+  virtual bool strongLts() const = 0;
   // local step with the LTS face buffers (the half-step time integral needs one more tile)
   virtual cudaError_t localLts(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the same without half-step integrals, for elements without a smaller neighbour (no extra tile)
@@ -57,11 +57,6 @@ class KernelSet {
   // GTS face projections leave the local kernel mixed with the reader's flux solver (fsLR)
   virtual bool premix() const = 0;
   virtual int fsPairStride() const = 0;
-  // room for the characteristic rows beside the pre-mixing buffers
-  virtual bool charMix() const = 0;
-  // the LTS local kernels mix face projections through the rank-3 factors of the flux-solver pairs
-  // when fsLR holds them (StepArgsRaw::fsChar; both of their tiles of characteristic rows fit)
-  virtual bool charMixLts() const = 0;
   virtual cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the neighbour step over the buffers the LTS local kernels wrote (pre-mixed where those
   // kernels have room for it)

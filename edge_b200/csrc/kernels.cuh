@@ -54,10 +54,8 @@ struct StepArgs {
   // elastic GTS (Geo::premix): per element face the element's own flux solver fsE[0] and the one
   // its face reader applies (fsE[1] of the face neighbour at its face, or the element's own for a
   // free surface; zeros for outflow) in T, each padded to 16 bytes (Geo::FSP): [nEl][4][2][FSP];
-  // null: gathered through the connectivity. fsChar: fsLR holds the characteristic factors of
-  // those pairs instead (LTS, Geo::charMixLts: V [9][4], then per quantity {U0[q][0..2], U1[q][0..2], 0, 0})
+  // null: gathered through the connectivity
   const T *fsLR;
-  int fsChar;
   // strong-form GTS steps (step.cuh): the coefficients of the elements, null for the
   // kernels of this file; per face the packed (neighbour * 4 + its face) * 4 + orientation or
   // 0xffffffff; the elements' own characteristics; face then holds those they
@@ -356,22 +354,7 @@ struct Geo {
   static constexpr size_t fsExtraOff = srcOff + srcBytes;
   static constexpr size_t tilesOff = (fsExtraOff + fsLocalBytes + 15) / 16 * 16;
   static constexpr bool projSplit = srcSplit && tilesOff + 2 * nS0 * sizeof(T) <= localBudget;
-  // characteristic mix (elastic GTS, pre-mixing): the two flux solvers a face projection P meets
-  // -- fsE[0] of the element and the reader's fsE[1] -- stacked (18 x 9) have rank 3, the three
-  // waves that leave the element through the face: [fsE0; fsE1] = [U0; U1] V^T. The nine warps
-  // first compute the three characteristic rows W = V^T P (a four-mode chunk each), then every
-  // warp its two output rows from W: 3 x 9 + 2 x 9 x 3 products per face mode instead of 2 x 81.
-  // W [3][32][SF] lives in X behind the face rows it holds during the faces, or behind the
-  // flux-solver buffers
-  static constexpr size_t nW = size_t(3) * 32 * SF;
-  static constexpr bool wInX = nW <= nX - nS0;
-  static constexpr bool charMix =
-      premix && (F + 3) / 4 <= 9 && (wInX || smemLocal + premixBytes + nW * sizeof(T) <= localBudget);
-  // LTS local kernels: the characteristic rows (and, in mode 2, those of the half-step projections)
-  // behind X's face rows, where both tiles fit there
-  static constexpr bool w2InX = 2 * nW <= nX - nS0;
-  static constexpr size_t smemLocalGts = premix      ? smemLocal + premixBytes +
-                                                      (charMix && !wInX ? nW * sizeof(T) : 0)
+  static constexpr size_t smemLocalGts = premix      ? smemLocal + premixBytes
                                          : projSplit ? tilesOff + 2 * nS0 * sizeof(T)
                                          : srcSplit  ? srcOff + srcBytes
                                          : fsLocal  ? smemLocal + fsLocalBytes + (coefSmem ? coefBytes : 0)
@@ -396,7 +379,6 @@ struct Geo {
   // the LTS local kernel without half-step integrals (mode 1)
   static constexpr size_t smemLocalSums = smemLocal + (premixLts ? premixBytes : 0);
   static constexpr bool ltsOk = tiSmem && smemLocalLts <= 227 * 1024;
-  static constexpr bool charMixLts = premixLts && charMix && ltsOk && w2InX;
   // neighbour kernel: a ring of NSN slots, each [9][32][SF] face rows and, for E <= 4, the E
   // elements' flux-solver blocks (81 + 54 doubles); as many slots (2..4) as fit the shared memory
   // of minCtasNeigh CTAs per SM (228 KB, 1 KB reserved per CTA)
@@ -856,22 +838,6 @@ __device__ __forceinline__ void faceMix2(const T *S0, int l, const T (&fr)[9], c
   }
 }
 
-// one mix of the characteristic rows: h[j] = sum_k u[k] W[k][j] for j < F (u: three values)
-template <typename T, int F, int SF>
-__device__ __forceinline__ void charMixOne(const T *Wt, int l, const T *u, T *h) {
-  const T u0 = u[0], u1 = u[1], u2 = u[2];
-#pragma unroll
-  for (int j0 = 0; j0 < F; j0 += 4) {
-    T w0[4], w1[4], w2[4];
-    ld4<T>(rowPtr<T, SF>(Wt, 0, l) + j0, w0);
-    ld4<T>(rowPtr<T, SF>(Wt, 1, l) + j0, w1);
-    ld4<T>(rowPtr<T, SF>(Wt, 2, l) + j0, w2);
-#pragma unroll
-    for (int v = 0; v < 4; v++)
-      if (j0 + v < F) h[j0 + v] = fmaT(u2, w2[v], fmaT(u1, w1[v], u0 * w0[v]));
-  }
-}
-
 // the flux-solver blocks of face FA of group g's elements (pre-mixed projections) into buf
 // [E][2][FSP]: 16-byte copies from fsLR, or (without it) loads gathered through the connectivity
 // and stored in T, visible after the next barrier like the copies
@@ -879,83 +845,13 @@ template <typename T>
 struct MixFs {
   T *buf;  // two buffers [2][E][2][FSP]
   int64_t g, nGroups;
-  T *w = nullptr;   // characteristic rows [3][32][SF] (Geo::charMix)
-  T *wh = nullptr;  // those of the half-step projections (LTS mode 2, Geo::charMixLts)
 };
 
-// characteristic rows of a face (Geo::charMix), first half: warp q < ceil(F / 4) computes modes
-// [4q, 4q + 4) of W[k] = sum_i V[i][k] S0[i] (k < 3) into Wt; fb = this lane's element's factors
-// (V [9][4] first). Modes past F read whatever the row holds there and count as zero.
-template <typename T, int F, int SF>
-__device__ __forceinline__ void charRows(const T *S0, const T *fb, int q, int l, T *Wt) {
-  if (q >= (F + 3) / 4) return;
-  const int j0 = 4 * q;
-  T w[3][4];
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-#pragma unroll
-    for (int u = 0; u < 4; u++) w[k][u] = T(0);
-#pragma unroll
-  for (int i = 0; i < 9; i++) {
-    T v[4], vk[4];
-    ld4<T>(rowPtr<T, SF>(S0, i, l) + j0, v);
-    ld4<T>(fb + 4 * i, vk);
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const T x = j0 + u < F ? v[u] : T(0);
-#pragma unroll
-      for (int k = 0; k < 3; k++) w[k][u] = fmaT(vk[k], x, w[k][u]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++) st4<T>(rowPtr<T, SF>(Wt, k, l) + j0, w[k]);
-}
-
-// second half: s[j] = sum_k uu[k] W[k][j] into registers, t[j] = sum_k uu[3 + k] W[k][j] written to
-// tRow[0, G) chunk by chunk; W is zero past F, so is t
-template <typename T, int F, int SF, int G>
-__device__ __forceinline__ void charMix2(const T *Wt, int l, const T *uu, T *s, T *tRow) {
-  T u[8];
-  {
-    T a[4], b[4];
-    ld4<T>(uu, a);
-    ld4<T>(uu + 4, b);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      u[i] = a[i];
-      u[4 + i] = b[i];
-    }
-  }
-#pragma unroll
-  for (int j0 = 0; j0 < F; j0 += 4) {
-    T w0[4], w1[4], w2[4], o[4], p[4];
-    ld4<T>(rowPtr<T, SF>(Wt, 0, l) + j0, w0);
-    ld4<T>(rowPtr<T, SF>(Wt, 1, l) + j0, w1);
-    ld4<T>(rowPtr<T, SF>(Wt, 2, l) + j0, w2);
-#pragma unroll
-    for (int v = 0; v < 4; v++) {
-      o[v] = fmaT(u[2], w2[v], fmaT(u[1], w1[v], u[0] * w0[v]));
-      p[v] = fmaT(u[5], w2[v], fmaT(u[4], w1[v], u[3] * w0[v]));
-    }
-#pragma unroll
-    for (int v = 0; v < 4; v++)
-      if (j0 + v < F) s[j0 + v] = o[v];
-    if (j0 + 4 <= G) {
-      st4<T>(tRow + j0, p);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 4; v++)
-        if (j0 + v < G) tRow[j0 + v] = p[v];
-    }
-  }
-}
-// CHAR: only the characteristic factors (the first 108 values: V [9][4], then {U0, U1} [9][8])
-template <typename T, int O, int R, int RM, int FA, bool CHAR = false>
+template <typename T, int O, int R, int RM, int FA>
 __device__ __forceinline__ void issueMixFs(const StepArgs<T> &a, T *buf, int64_t g, int64_t nGroups) {
   using G = Geo<T, O, R, RM>;
   constexpr int E = G::E, FSP = G::FSP, W = 16 / int(sizeof(T)), NC = FSP / W;
-  constexpr int NCP = CHAR ? 108 / W : 2 * NC;  // chunks copied per element face
-  static_assert(108 % W == 0 && 108 <= 2 * FSP, "factor entries of whole chunks within the pair stride");
+  constexpr int NCP = 2 * NC;  // chunks copied per element face
   if (g >= nGroups) return;
   if (a.fsLR) {
     for (int i = threadIdx.x; i < E * NCP; i += G::NT) {
@@ -1069,8 +965,7 @@ __device__ __forceinline__ int neighOri(const FaceMeta &m) {
 // projections of elements with a smaller neighbour (needs TIh)
 // pre-mixed projections (LTS 0, Geo::premix): S0alt is a tile free for this warp's own rows,
 // through which the mixed projection leaves as coalesced stores; mf the flux-solver buffers
-// CHAR: the pre-mixed projections mix through the characteristic factors in mf.buf (Geo::charMix)
-template <typename T, int O, int R, int RM, int FA, int LTS = 0, bool TAIL = true, bool CHAR = false>
+template <typename T, int O, int R, int RM, int FA, int LTS = 0, bool TAIL = true>
 __device__ __forceinline__ void localFace(const StepArgs<T> &a, const T *TI, T *S0, int q, int l, int64_t e,
                                           int r, bool valid, T *acc, T *upA, const T *TIh = nullptr,
                                           T *S0alt = nullptr, const MixFs<T> &mf = MixFs<T>{nullptr, 0, 0},
@@ -1145,34 +1040,21 @@ __device__ __forceinline__ void localFace(const StepArgs<T> &a, const T *TI, T *
     // the next face's blocks into the other buffer, whose readers (two faces back) all passed the
     // barrier; after the last face the next group's first
     if constexpr (FA < 3)
-      issueMixFs<T, O, R, RM, FA + 1, CHAR>(a, mf.buf + ((FA + 1) % 2) * (E * 2 * FSP), mf.g, mf.nGroups);
+      issueMixFs<T, O, R, RM, FA + 1>(a, mf.buf + ((FA + 1) % 2) * (E * 2 * FSP), mf.g, mf.nGroups);
     else
-      issueMixFs<T, O, R, RM, 0, CHAR>(a, mf.buf, mf.g + gridDim.x, mf.nGroups);
+      issueMixFs<T, O, R, RM, 0>(a, mf.buf, mf.g + gridDim.x, mf.nGroups);
     cpAsyncCommit();
     const T *fbE = mf.buf + (FA % 2) * (E * 2 * FSP) + (l / R) * (2 * FSP);
-    static_assert(!CHAR || (LTS == 0 ? G::charMix : G::charMixLts),
-                  "characteristic mix: configurations with room for its rows");
-    // the mixed projection t of this warp's row: through the characteristic rows of all warps'
-    // projections (CHAR; it leaves through this warp's own row of S0, which no warp reads after the
-    // second barrier), else through the pair blocks (through the warp's row of S0alt)
-    T *tile = CHAR ? S0 : S0alt;
+    // the mixed projection t of this warp's row, through the warp's row of S0alt
+    T *tile = S0alt;
     T *tRow = rowPtr<T, SF>(tile, q, l);
-    T fr1[CHAR ? 1 : 9];
-    if constexpr (CHAR) {
-      charRows<T, F, SF>(S0, fbE, q, l, mf.w);
-      // with half-step projections (LTS 2) their characteristic rows too
-      if constexpr (LTS == 2) charRows<T, F, SF>(ShF, fbE, q, l, mf.wh);
-      __syncthreads();
-      charMix2<T, F, SF, G::GF>(mf.w, l, fbE + 36 + q * 8, s, tRow);
-    } else {
-      T fr[9];
+    T fr[9], fr1[9];
 #pragma unroll
-      for (int i = 0; i < 9; i++) {
-        fr[i] = fbE[q * 9 + i];
-        fr1[i] = fbE[FSP + q * 9 + i];
-      }
-      faceMix2<T, F, SF, G::GF>(S0, l, fr, fr1, s, tRow);
+    for (int i = 0; i < 9; i++) {
+      fr[i] = fbE[q * 9 + i];
+      fr1[i] = fbE[FSP + q * 9 + i];
     }
+    faceMix2<T, F, SF, G::GF>(S0, l, fr, fr1, s, tRow);
     __syncwarp();
     if (ty != FT_OUTFLOW)
       storeRowsCoalesced<T, R, G::GF, SF>(tile, a.face + ((e * 4 + FA) * 9 + q) * int64_t(R * G::GF), q, l / R,
@@ -1193,10 +1075,7 @@ __device__ __forceinline__ void localFace(const StepArgs<T> &a, const T *TI, T *
         }
         if (LTS == 2 && half) {
           T h[F], t[F];
-          if constexpr (CHAR)
-            charMixOne<T, F, SF>(mf.wh, l, fbE + 36 + q * 8 + 3, h);
-          else
-            faceMix<T, F, SF>(ShF, l, fr1, h);
+          faceMix<T, F, SF>(ShF, l, fr1, h);
           const int64_t slot = int64_t(a.halfIdx[e]) * 4 + FA;
           stRowG<T, F>(gRow<T, R, G::GF>(a.faceHalf1, slot, 9, q, r), h);
           ldRow<T, F>(tRow, t);
@@ -1323,8 +1202,7 @@ __device__ __forceinline__ void facesSplit(const StepArgs<T> &a, const T *TI, T 
 
 // LTS as in localFace; mode 2 keeps the half-step integral in one more tile (one CTA per SM), mode
 // 1 runs on the elements of a time group without a smaller neighbour
-// CHAR (LTS): the mixes go through the characteristic factors
-template <typename T, int O, int R, int RM, int LTS, bool CHAR = false>
+template <typename T, int O, int R, int RM, int LTS>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O, R, RM>::minCtasLocal)
     kLocal(StepArgs<T> a) {
   using G = Geo<T, O, R, RM>;
@@ -1382,7 +1260,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         for (int m = 0; m < RM; m++)
           copyRows<T, R, G::GB, SB>(TIA, a.dofsA, a.elFirst + g0 * E + eo, RM * 6, m * 6 + q - 9, eo, r);
     }
-    if constexpr (PM) issueMixFs<T, O, R, RM, 0, CHAR>(a, fsb, g0, nGroups);
+    if constexpr (PM) issueMixFs<T, O, R, RM, 0>(a, fsb, g0, nGroups);
     if constexpr (FL) issueLocalFs<T, O, R, RM, 0>(a, fsl, g0, nGroups);
     if constexpr (PSP) {
       issueLocalFs<T, O, R, RM, 1>(a, fsl + E * G::NFL, g0, nGroups);
@@ -1529,10 +1407,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
     }
     // local surface integral (SurfIntVanilla::local, SurfIntVanilla.hpp:212-262) + face projections
     if constexpr (AS) {
-      // characteristic rows: behind the face rows of X, or behind the flux-solver buffers
-      T *const wTile =
-          CHAR ? (G::wInX ? X + G::nS0 : reinterpret_cast<T *>(smem + G::smemLocal + G::premixBytes)) : nullptr;
-      const MixFs<T> mf{fsb, g, nGroups, wTile, (CHAR && LTS == 2) ? X + G::nS0 + G::nW : nullptr};
+      const MixFs<T> mf{fsb, g, nGroups};
       const LocalFs lf{fsl, g, nGroups};
       if constexpr (PSP) {
         T *const tiles[4] = {S0, X, reinterpret_cast<T *>(smem + G::tilesOff),
@@ -1547,12 +1422,11 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         issueLocalFs<T, O, R, RM, 3>(a, fsExtra + E * G::NFL, gn, nGroups);
         cpAsyncCommit();
       } else {
-        localFace<T, O, R, RM, 0, LTS, false, CHAR>(a, TI, S0, q, l, ev, r, valid, acc, upA, TIh, X, mf, Sh, lf);
-        localFace<T, O, R, RM, 1, LTS, false, CHAR>(a, TI, X, q, l, ev, r, valid, acc, upA, TIh, S0, mf, Sh, lf);
-        localFace<T, O, R, RM, 2, LTS, false, CHAR>(a, TI, S0, q, l, ev, r, valid, acc, upA, TIh, X, mf, Sh, lf);
-        // the barrier after the last face orders its readers of X (and of the characteristic rows
-        // behind its face rows) before the next group writes X
-        localFace<T, O, R, RM, 3, LTS, true, CHAR>(a, TI, X, q, l, ev, r, valid, acc, upA, TIh, S0, mf, Sh, lf);
+        localFace<T, O, R, RM, 0, LTS, false>(a, TI, S0, q, l, ev, r, valid, acc, upA, TIh, X, mf, Sh, lf);
+        localFace<T, O, R, RM, 1, LTS, false>(a, TI, X, q, l, ev, r, valid, acc, upA, TIh, S0, mf, Sh, lf);
+        localFace<T, O, R, RM, 2, LTS, false>(a, TI, S0, q, l, ev, r, valid, acc, upA, TIh, X, mf, Sh, lf);
+        // the barrier after the last face orders its readers of X before the next group writes X
+        localFace<T, O, R, RM, 3, LTS, true>(a, TI, X, q, l, ev, r, valid, acc, upA, TIh, S0, mf, Sh, lf);
       }
       if constexpr (SS)
         if (q < 6) addSrcRows<T, B, SB>(srcBuf, q, l, acc);
@@ -2036,7 +1910,7 @@ __device__ __forceinline__ void recvAll(T *X, T *TI, T *XA, T *TIA, int q, int l
 // (step.cuh)
 template <typename T, int O, int R>
 struct SGeo;
-template <typename T, int O, int R>
+template <typename T, int O, int R, bool LTS>
 __device__ __forceinline__ void liftRow(const StepArgs<T> &a, const T *in, T *wt, int t, int l, int64_t e, int r,
                                         bool valid);
 template <typename T, int O, int R, int RM>
@@ -2078,7 +1952,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
   }
   if (a.faceIn) {
     static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
-    for (int t = q; t < 12; t += G::NW) liftRow<T, O, R>(a, a.faceIn, X, t, l, ev, r, valid);
+    for (int t = q; t < 12; t += G::NW) liftRow<T, O, R, false>(a, a.faceIn, X, t, l, ev, r, valid);
     __syncthreads();
     liftApply<T, O, R>(X, FacU<T, O, R, RM>{facPtr<T, O, R, RM>(a.fac, ev), q}, l, v);
     __syncthreads();

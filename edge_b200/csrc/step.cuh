@@ -222,7 +222,7 @@ __device__ __forceinline__ void rowFinish(T *wt, int t, uint32_t gs, int l, T *v
 #pragma unroll
   for (int c = 0; c < G::CW; c++) stChunk<T>(faceChunk<T, O, R>(wt, t, l, c), v + c * G::W);
 }
-template <typename T, int O, int R>
+template <typename T, int O, int R, bool LTS>
 __device__ __forceinline__ void liftRow(const StepArgs<T> &a, const T *in, T *wt, int t, int l, int64_t e, int r,
                                         bool valid) {
   using G = SGeo<T, O, R>;
@@ -230,7 +230,16 @@ __device__ __forceinline__ void liftRow(const StepArgs<T> &a, const T *in, T *wt
   const uint32_t gs = valid ? __ldg(a.gath + e * 4 + t / 3) : kNoNeighbour;
   rowOwn<T, O, R>(a, t, e, r, valid, v);
   if (gs != kNoNeighbour) {
-    const T *nb = in + charRow<T, O, R>(gs >> 2, t % 3, r);
+    int64_t slot = gs >> 2;
+    if constexpr (LTS) {
+      // what the neighbour wrote over this element's step: its two-step sum, or its half-step rows
+      const int rel = a.ltsRel[e * 4 + t / 3];
+      if (rel != LTS_EQ) {
+        in = rel == LTS_GT ? a.faceSum : a.firstTs ? a.faceHalf1 : a.faceHalf2;
+        slot = int64_t((rel == LTS_GT ? a.sumIdx : a.halfIdx)[gs >> 4]) * 4 + (gs >> 2 & 3);
+      }
+    }
+    const T *nb = in + charRow<T, O, R>(slot, t % 3, r);
 #pragma unroll
     for (int c = 0; c < G::CW; c++) ldChunk<T>(nb + c * (R * G::W), x + c * G::W);
     turnRow<O, T>(gs & 3u, x, v);
@@ -404,9 +413,10 @@ __device__ __forceinline__ void projectFace(T *t, const T *ti, const T *acc, T d
 }
 
 // derivatives D .. O-1 (see CkStep): acc accumulates Q*, ti the time integral of the first NK modes
-template <typename T, int O, int R, int D>
+// (H: th that over the first half of the step, for LTS)
+template <typename T, int O, int R, int D, bool H>
 __device__ __forceinline__ void ckStrong(T *X, T *XP, int q, int l, const int (&cols)[3], const T (&cs)[3][3], T dt,
-                                         T sca, T *acc, T *ti) {
+                                         T sca, T scaH, T *acc, T *ti, T *th) {
   if constexpr (D < O) {
     using G = SGeo<T, O, R>;
     constexpr int NN = nModes(O - D);
@@ -422,19 +432,23 @@ __device__ __forceinline__ void ckStrong(T *X, T *XP, int q, int l, const int (&
     if constexpr (D + 1 < O) stRow<T, NN>(rowPtr<T, SO>(out, q, l), d);
     // sca = dt^D / D!
     const T scb = sca * dt / T(D + 1);
+    // scaH = (dt / 2)^D / D!
+    const T scbH = H ? scaH * (dt * T(0.5)) / T(D + 1) : T(0);
 #pragma unroll
     for (int n = 0; n < NN; n++) {
+      if constexpr (H) th[n] = fmaT(scbH, d[n], D == 1 ? (dt * T(0.5)) * acc[n] : th[n]);
       ti[n] = fmaT(scb, d[n], D == 1 ? dt * acc[n] : ti[n]);
       acc[n] = fmaT(sca, d[n], acc[n]);
     }
     if constexpr (D + 1 < O) __syncthreads();
-    ckStrong<T, O, R, D + 1>(X, XP, q, l, cols, cs, dt, scb, acc, ti);
+    ckStrong<T, O, R, D + 1, H>(X, XP, q, l, cols, cs, dt, scb, scbH, acc, ti, th);
   }
 }
 
 // characteristics of one 16-byte chunk c of face f's modes (its projections in tile p): the element's
 // own rows and its neighbour's, to device memory
-template <typename T, int O, int R>
+// LTS: also added up over the two steps of a pair for a larger neighbour (faceSum)
+template <typename T, int O, int R, int LTS = 0>
 __device__ __forceinline__ void charTask(const StepArgs<T> &a, const T *p, const T *V, int f, int c, int l, int64_t e,
                                          int r, bool valid) {
   using G = SGeo<T, O, R>;
@@ -470,13 +484,66 @@ __device__ __forceinline__ void charTask(const StepArgs<T> &a, const T *p, const
     stChunk<T>(a.wOwn + ownRow<T, O, R>(e, 3 * f + k, r) + c * (32 * G::W), w[k]);
     stChunk<T>(a.face + charRow<T, O, R>(e * 4 + f, k, r) + c * (R * G::W), w[3 + k]);
   }
+  if constexpr (LTS > 0) {
+    if (a.ltsFlags[e] & LTS_HAS_LARGER) {
+      const int64_t slot = int64_t(a.sumIdx[e]) * 4 + f;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        T *p2 = a.faceSum + charRow<T, O, R>(slot, k, r) + c * (R * G::W);
+        T x[G::W];
+        ldChunk<T>(p2, x);
+#pragma unroll
+        for (int u = 0; u < G::W; u++) x[u] = a.firstTs ? w[3 + k][u] : x[u] + w[3 + k][u];
+        stChunk<T>(p2, x);
+      }
+    }
+  }
+}
+
+// The neighbour's rows of the half-step projections in tile p, for elements with a smaller neighbour:
+// faceHalf1 over the first half of the step, faceHalf2 over the second (what this thread's charTask
+// wrote for the whole step less the first half)
+template <typename T, int O, int R>
+__device__ __forceinline__ void halfTask(const StepArgs<T> &a, const T *p, const T *V, int f, int c, int l, int64_t e,
+                                         int r, bool half) {
+  using G = SGeo<T, O, R>;
+  T w[3][G::W];
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+#pragma unroll
+    for (int i = 0; i < G::W; i++) w[k][i] = T(0);
+#pragma unroll 3
+  for (int i = 0; i < 9; i++) {
+    T x[G::W], v[8];
+    ldChunk<T>(faceChunk<T, O, R>(const_cast<T *>(p), i, l, c), x);
+#pragma unroll
+    for (int k = 0; k < 8; k += G::W) ldChunk<T>(V + (i * 8 + k) * G::E, v + k);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int u = 0; u < G::W; u++) w[k][u] = fmaT(v[3 + k], x[u], w[k][u]);
+  }
+  if (!half) return;
+  const int64_t slot = int64_t(a.halfIdx[e]) * 4 + f;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int64_t o = charRow<T, O, R>(slot, k, r) + c * (R * G::W);
+    T x[G::W];
+    ldChunk<T>(a.face + charRow<T, O, R>(e * 4 + f, k, r) + c * (R * G::W), x);
+    stChunk<T>(a.faceHalf1 + o, w[k]);
+#pragma unroll
+    for (int u = 0; u < G::W; u++) x[u] -= w[k][u];
+    stChunk<T>(a.faceHalf2 + o, x);
+  }
 }
 
 // One GTS step of elements [elFirst, elFirst + elCount) up to their surface integrals: the pending
 // characteristics of the previous step (faceIn and wOwn, none when faceIn is null) complete the DOF
 // rows, the recursion updates them, and this step's characteristics leave in face and wOwn.
-template <typename T, int O, int R>
-__global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(const StepArgs<T> a) {
+// LTS 1, 2: the local step of a time group (rate-2 local time stepping; nothing is pending then): the
+// neighbours' rows also summed over two steps, and with 2 the half-step rows
+template <typename T, int O, int R, int LTS = 0>
+__global__ void __launch_bounds__(SGeo<T, O, R>::NT, LTS == 2 ? 1 : SGeo<T, O, R>::ctas) kStep(const StepArgs<T> a) {
   using G = SGeo<T, O, R>;
   constexpr int B = G::B, E = G::E, SB = G::SB;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -487,6 +554,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
   T *const bufV = reinterpret_cast<T *>(smem + G::offV);
   const int64_t nGroups = (a.elCount + E - 1) / E;
   // elements of group g
+  const bool pending = LTS == 0 && a.faceIn;
   const auto inGroup = [&](int64_t g) { return int(min(a.elCount - g * E, int64_t(E))); };
   const T dt0 = T(a.dt);
   uint32_t gs0 = kNoNeighbour, gs1 = kNoNeighbour;
@@ -500,7 +568,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     // pending characteristics: warp q takes rows q and (q < 3) q + 9; gather entries and own parts of
     // the current group
     const int t1 = q < 3 ? q + 9 : q;
-    const bool pend = a.faceIn && g * E + eo < a.elCount;
+    const bool pend = pending && g * E + eo < a.elCount;
     const int64_t e = pend ? a.elFirst + g * E + eo : a.elFirst;
     if (pend) {
       gs0 = __ldg(a.gath + e * 4 + q / 3);
@@ -523,7 +591,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     const bool valid = g * E + eo < a.elCount;
     const int64_t e = valid ? a.elFirst + g * E + eo : a.elFirst;
     const int64_t gn = g + gridDim.x;
-    const T dt = a.grpDt ? T(a.grpDt[g]) : dt0;
+    const T dt = LTS == 0 && a.grpDt ? T(a.grpDt[g]) : dt0;
     const T *const facE = facPtr<T, O, R, 0>(a.fac, e);
     const T *const cU = G::smemU ? bufU + eo * G::W : facE;
     const T *const cV = G::smemV ? bufV + eo * G::W : facE + FacL<0>::V * E;
@@ -541,7 +609,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     const int64_t en = validN ? a.elFirst + gn * E + eo : a.elFirst;
     cpAsyncWait<0>();
     __syncwarp();
-    if (a.faceIn) {
+    if (pending) {
       rowFinish<T, O, R>(XP, q, gs0, l, w0);
       if (q < 3) rowFinish<T, O, R>(XP, t1, gs1, l, w1);
       gs0 = gs1 = kNoNeighbour;
@@ -560,7 +628,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     } else {
       ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, e, 9, q, r), acc, valid);
     }
-    if (a.faceIn) {
+    if (pending) {
       if constexpr (G::smemU)
         liftApply<T, O, R>(XP, su, l, acc);
       else
@@ -581,8 +649,8 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     if constexpr (G::smemU) issueFac<T, O, R, 0>(a, bufU, 0, FacL<0>::V, gn, nGroups);
     if constexpr (!G::smemV) prefetchFac<T, O, R, 0>(a, G::smemU ? FacL<0>::V : 0, FacL<0>::len, gn, nGroups);
     cpAsyncCommit();
-    T ti[G::NK];
-    ckStrong<T, O, R, 1>(X, XP, q, l, cols, cs, dt, dt, acc, ti);
+    T ti[G::NK], th[LTS == 2 ? G::NK : 1];
+    ckStrong<T, O, R, 1, LTS == 2>(X, XP, q, l, cols, cs, dt, dt, dt * T(0.5), acc, ti, th);
     if (a.tDofs && valid) {
       T t[B];
 #pragma unroll
@@ -614,7 +682,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     cpAsyncWait<2>();
     __syncthreads();
     // (every warp is past the recursion: the tile of odd derivatives takes the next group's rows)
-    if (a.faceIn) {
+    if (pending) {
       rowNeighbour<T, O, R>(a.faceIn, XP, q, gs0, l);
       if (q < 3) rowNeighbour<T, O, R>(a.faceIn, XP, t1, gs1, l);
     }
@@ -622,7 +690,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
     if constexpr (G::NFR == 2) {
       for (int t = q; t < 2 * G::CW; t += 9) {
         const int i = t / G::CW, c = t - i * G::CW;
-        charTask<T, O, R>(a, X + i * G::nF, cV + (i + 2) * 72 * E, i + 2, c, l, e, r, valid);
+        charTask<T, O, R, LTS>(a, X + i * G::nF, cV + (i + 2) * 72 * E, i + 2, c, l, e, r, valid);
       }
       __syncthreads();
       projectFace<T, O, R, 0>(X, ti, acc, dt, q, l);
@@ -630,12 +698,32 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
       __syncthreads();
     }
     // (both arrays are set on every path: they do not live through the group)
-    rowOwn<T, O, R>(a, q, en, r, validN && a.faceIn, w0);
-    rowOwn<T, O, R>(a, t1, en, r, validN && a.faceIn && q < 3, w1);
+    rowOwn<T, O, R>(a, q, en, r, validN && pending, w0);
+    rowOwn<T, O, R>(a, t1, en, r, validN && pending && q < 3, w1);
     for (int t = q; t < G::NFR * G::CW; t += 9) {
       const int i = t / G::CW, c = t - i * G::CW;
       const int f = G::NFR == 4 ? (i + 2) & 3 : i;
-      charTask<T, O, R>(a, X + i * G::nF, cV + f * 72 * E, f, c, l, e, r, valid);
+      charTask<T, O, R, LTS>(a, X + i * G::nF, cV + f * 72 * E, f, c, l, e, r, valid);
+    }
+    if constexpr (LTS == 2) {
+      const bool half = valid && (a.ltsFlags[e] & LTS_HAS_SMALLER);
+      if (__any_sync(0xffffffffu, half)) {  // (the same in every warp)
+#pragma unroll
+        for (int p = 0; p < 4; p += G::NFR) {
+          __syncthreads();
+          if (p == 0) projectPair<T, O, R>(X, X + G::nF, th, acc, dt * T(0.5), q, l);
+          if (p + G::NFR == 4) {
+            projectFace<T, O, R, 0>(X + (2 - p) * G::nF, th, acc, dt * T(0.5), q, l);
+            projectFace<T, O, R, 1>(X + (3 - p) * G::nF, th, acc, dt * T(0.5), q, l);
+          }
+          __syncthreads();
+          for (int t = q; t < G::NFR * G::CW; t += 9) {
+            const int i = t / G::CW, c = t - i * G::CW;
+            const int f = (i + p + 2) & 3;
+            halfTask<T, O, R>(a, X + i * G::nF, cV + f * 72 * E, f, c, l, e, r, half);
+          }
+        }
+      }
     }
   }
   cpAsyncWait<0>();
@@ -643,7 +731,7 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctas) kStep(
 
 // The pending surface integrals on their own (the closing half of a step): face holds the
 // characteristics written for the elements by their neighbours, wOwn their own.
-template <typename T, int O, int R>
+template <typename T, int O, int R, bool LTS = false>
 __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctasLift) kLift(const StepArgs<T> a) {
   using G = SGeo<T, O, R>;
   constexpr int B = G::B, E = G::E, SB = G::SB;
@@ -667,8 +755,8 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctasLift) kL
 #pragma unroll
       for (int f = 0; f < 4; f++) su(f, ru.u[f]);
     }
-    liftRow<T, O, R>(a, a.face, wt, q, l, e, r, valid);
-    if (q < 3) liftRow<T, O, R>(a, a.face, wt, q + 9, l, e, r, valid);
+    liftRow<T, O, R, LTS>(a, a.face, wt, q, l, e, r, valid);
+    if (q < 3) liftRow<T, O, R, LTS>(a, a.face, wt, q + 9, l, e, r, valid);
     cpAsyncWait<0>();
     __syncthreads();
     T acc[B];

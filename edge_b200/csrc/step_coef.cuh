@@ -7,7 +7,8 @@
 namespace edge_b200 {
 
 // Nine lanes share a face, lane a its row a of the 9 x 9 solvers; what they exchange goes through this
-// (a thread per face keeps its matrices in local memory: 6.2 against 0.6 ms for 72,864 elements).
+// (a thread per face keeps its matrices in local memory: 6.2 against 2.2 ms for 72,864 elements, each with
+// its launch and the check read back).
 struct FaceTeam {
   double S[9][9], N[9][9], U[9][3], V0[9][3], red[9];
 };
@@ -108,9 +109,9 @@ __device__ __forceinline__ double rowBasis(FaceTeam &t, int a, double (&S)[9], d
   return res;
 }
 
-// Two items per face: part 0: V1 of the face's reader (a function of the reader's fsE[1] alone, so that
-// parts of a partition agree on it); part 1: U and V0 of the face, and with face 0 the element's other
-// coefficients. Counts lanes that find their face's solvers not of rank 3 in this form in *bad.
+// Per face: V1 of its reader (a function of the reader's fsE[1] alone, so that parts of a partition agree
+// on it), U and V0; with face 0 the element's other coefficients. Counts lanes that find solvers not of
+// rank 3 in this form in *bad. Values leave as whole 16-byte chunks.
 template <typename T>
 __global__ void __launch_bounds__(kBuildWarps * 32)
     kBuildStep(const double *fsE, const double *starE, const double *fsA, const double *starA, const double *srcA,
@@ -119,12 +120,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
   __shared__ FaceTeam teams[kBuildWarps][kTeams + 1];
   const int l = threadIdx.x & 31, team = l / 9, a = l - 9 * team;  // (lanes 27 .. 31 repeat the last team's item)
   FaceTeam &t = teams[threadIdx.x >> 5][team];
-  const int64_t items = nEl * 8, stride = int64_t(gridDim.x) * kBuildWarps * kTeams;
+  const int64_t items = nEl * 4, stride = int64_t(gridDim.x) * kBuildWarps * kTeams;
   for (int64_t i0 = (int64_t(blockIdx.x) * kBuildWarps + (threadIdx.x >> 5)) * kTeams; i0 < items; i0 += stride) {
     const int64_t i = min(i0 + min(team, kTeams - 1), items - 1);
     const bool mine = team < kTeams && i0 + team < items;
-    const int part = int(i & 1);
-    const int64_t ef = i >> 1, e = ef >> 2;
+    const int64_t ef = i, e = ef >> 2;
     const int f = int(ef & 3), ty = faType[ef];
     // value k of the element's coefficients (16-byte chunks interleaved over E elements)
     constexpr int W = 16 / int(sizeof(T));
@@ -132,17 +132,40 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
     const int V = (rm ? FacL<3>::src + 12 * rm : FacL<0>::V) + f * 72;
     const int len = V - f * 72 + 288;
     T *const fe = fac + (e / E) * (int64_t(len) * E) + (e % E) * W;
-    const auto put = [&](int k, double v) {
-      if (mine) fe[k / W * (E * W) + k % W] = T(v);
+    // four values from k on (a multiple of four)
+    const auto put4 = [&](int k, double v0, double v1, double v2, double v3) {
+      if (!mine) return;
+      T *p = fe + k / W * (E * W);
+      if constexpr (W == 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(float(v0), float(v1), float(v2), float(v3));
+      } else {
+        *reinterpret_cast<double2 *>(p) = make_double2(v0, v1);
+        *reinterpret_cast<double2 *>(p + E * W) = make_double2(v2, v3);
+      }
     };
     const bool inner = ty == FT_INNER;
     const int64_t n = inner ? elFaEl[ef] : e;
     const int fo = inner ? fId[ef] : f;
-    // this lane's rows: M what the basis comes from, N the own side
-    // (part 0: the neighbour reads this element's projection at its own face, through its fsE[1] there)
-    const double *pm = fsE + (nEl * 4 + (part == 0 ? n * 4 + fo : ef)) * 81 + a * 9;
-    const double *pn = fsE + ef * 81 + a * 9;
-    double M[9], N[9], add[9];
+    // V1: the neighbour reads this element's projection at its own face, through its fsE[1] there
+    double v1[3] = {0, 0, 0}, M[9], N[9], S[9], Q[3][9];
+    bool off;
+    {
+      const double *p = fsE + (nEl * 4 + n * 4 + fo) * 81 + a * 9;
+#pragma unroll
+      for (int j = 0; j < 9; j++) M[j] = __ldg(p + j);
+      const Scales s1 = scales(t, a, M);
+#pragma unroll
+      for (int j = 0; j < 9; j++) S[j] = M[j] / (s1.r(a) * s1.c(j));
+      off = rowBasis(t, a, S, Q) > kRankTol2 && inner;
+#pragma unroll
+      for (int j = 0; j < 9; j++)
+        if (j == a && inner)
+#pragma unroll
+          for (int k = 0; k < 3; k++) v1[k] = s1.c(j) * Q[k][j];
+    }
+    // this lane's rows: M what U's basis comes from, N the own side
+    const double *pm = fsE + (nEl * 4 + ef) * 81 + a * 9, *pn = fsE + ef * 81 + a * 9;
+    double add[9];
 #pragma unroll
     for (int j = 0; j < 9; j++) {
       M[j] = __ldg(pm + j);
@@ -153,7 +176,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
     const Scales sc = inner ? sc1 : sc0;
     const double nrm[3] = {f == 2 ? -1.0 : f == 3 ? 1.0 : 0.0, f == 1 ? -1.0 : f == 3 ? 1.0 : 0.0,
                            f == 0 ? -1.0 : f == 3 ? 1.0 : 0.0};
-    if (part == 1) {
+    {
       // N = fsE[0] + sum_d n_fd star_d (+ fsE[1] of a free surface, which reads this element)
       const double *st = starE + e * 72;
       double sd[3][3];
@@ -178,27 +201,16 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
       }
       if (f == 0) {
         // the star rows along the derivative directions of the generated products
-#pragma unroll
-        for (int k = 0; k < 12; k++) put(oStar + a * 12 + k, k < 9 ? sd[k < 9 ? k / 3 : 0][k % 3] : 0.0);
+        put4(oStar + a * 12, sd[0][0], sd[0][1], sd[0][2], sd[1][0]);
+        put4(oStar + a * 12 + 4, sd[1][1], sd[1][2], sd[2][0], sd[2][1]);
+        put4(oStar + a * 12 + 8, sd[2][2], 0, 0, 0);
       }
-    } else if (mine && a == 0) {
-      gath[ef] = inner ? uint32_t((n * 4 + fo) * 4 + kFacePerm[order - 2][fo][f][vId[ef]]) : kNoNeighbour;
     }
-    double S[9], Q[3][9];
+    if (mine && a == 0)
+      gath[ef] = inner ? uint32_t((n * 4 + fo) * 4 + kFacePerm[order - 2][fo][f][vId[ef]]) : kNoNeighbour;
 #pragma unroll
     for (int j = 0; j < 9; j++) S[j] = M[j] = M[j] / (sc.r(a) * sc.c(j));
-    bool off = rowBasis(t, a, S, Q) > kRankTol2;
-    if (part == 0) {
-#pragma unroll
-      for (int j = 0; j < 9; j++)
-        if (j == a) {
-#pragma unroll
-          for (int k = 0; k < 3; k++) put(V + 8 * j + 3 + k, inner ? sc.c(j) * Q[k][j] : 0.0);
-          put(V + 8 * j + 6, 0);
-          put(V + 8 * j + 7, 0);
-        }
-      off = off && inner;
-    }
+    off = rowBasis(t, a, S, Q) > kRankTol2 || off;
     // U (scaled rows), then V0 from U V0^T = N: every lane holds U and solves for its own column
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -206,9 +218,8 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
 #pragma unroll
       for (int j = 0; j < 9; j++) u += M[j] * Q[k][j];
       t.U[a][k] = u;
-      if (part == 1) put(f * 4 * rows + a * 4 + k, sc.r(a) * u);
     }
-    if (part == 1) put(f * 4 * rows + a * 4 + 3, 0);
+    put4(f * 4 * rows + a * 4, sc.r(a) * t.U[a][0], sc.r(a) * t.U[a][1], sc.r(a) * t.U[a][2], 0);
 #pragma unroll
     for (int j = 0; j < 9; j++) t.N[a][j] = N[j] / sc.r(a);
     __syncwarp();
@@ -261,22 +272,19 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
       x[k] = Rm[k][k] > 0 ? v / Rm[k][k] : 0.0;
     }
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      t.V0[a][k] = x[k];
-      if (part == 1) put(V + 8 * a + k, x[k]);
-    }
+    for (int k = 0; k < 3; k++) t.V0[a][k] = x[k];
+    put4(V + 8 * a, x[0], x[1], x[2], v1[0]);
+    put4(V + 8 * a + 4, v1[1], v1[2], 0, 0);
     // residuals against the largest entry of the column's kind
     const double top = sc.c(a);
-    if (part == 1) off = off || !(res <= kRankTol2 * top * top);
+    off = off || !(res <= kRankTol2 * top * top);
     __syncwarp();
-    // (the teams of a warp may hold different parts: all of them pass the warp barriers, and part 0
-    // writes nothing here)
     if (rm) {
       // anelastic rows (lanes 0 .. 5): UA over the same basis, and the same V0 has to give
       // fsA[0]' = fsA[0] + sum_d n_fd starA_d
       const int s = a < 6 ? a : 0;
       const double *f0 = fsA + ef * 54 + s * 9, *f1 = fsA + (nEl * 4 + ef) * 54 + s * 9, *sa = starA + e * 27;
-      double na[9], ma[9], mS = 0, mV = 0;
+      double na[9], ma[9], mS = 0, mV = 0, sda[6];
 #pragma unroll
       for (int j = 0; j < 9; j++) {
         na[j] = __ldg(f0 + j);
@@ -298,26 +306,24 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
 #pragma unroll
         for (int j = 0; j < 9; j++)
           if (j == col) na[j] += nrm[0] * v[0] + nrm[1] * v[1] + nrm[2] * v[2];
-        if (part == 1 && f == 0 && a < 6)
 #pragma unroll
-          for (int d = 0; d < 3; d++)
-            put(FacL<3>::starA + s * 8 + 2 * d + i2, kStarDir[0][d] * v[0] + kStarDir[1][d] * v[1] + kStarDir[2][d] * v[2]);
+        for (int d = 0; d < 3; d++)
+          sda[2 * d + i2] = kStarDir[0][d] * v[0] + kStarDir[1][d] * v[1] + kStarDir[2][d] * v[2];
       }
 #pragma unroll
       for (int j = 0; j < 9; j++) {
         if (ty == FT_FREE) na[j] += ma[j];
         if (!inner) ma[j] = na[j];
       }
-      if (part == 1 && a < 6) {
+      if (a < 6) {
         double u[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
           u[k] = 0;
 #pragma unroll
           for (int j = 0; j < 9; j++) u[k] += ma[j] / sc.c(j) * Q[k][j];
-          put(f * 4 * rows + (9 + s) * 4 + k, u[k]);
         }
-        put(f * 4 * rows + (9 + s) * 4 + 3, 0);
+        put4(f * 4 * rows + (9 + s) * 4, u[0], u[1], u[2], 0);
 #pragma unroll
         for (int j = 0; j < 9; j++) {
           const double tol = 1e-9 * (j < 6 ? topS : topV);
@@ -330,9 +336,12 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
           off = off || !(fabs(r1) <= tol) || !(fabs(r0) <= tol);
         }
         if (f == 0) {
-          put(FacL<3>::starA + s * 8 + 6, 0);
-          put(FacL<3>::starA + s * 8 + 7, 0);
-          for (int k = s; k < 12 * rm; k += 6) put(FacL<3>::src + k, srcA[e * 12 * rm + k]);
+          put4(FacL<3>::starA + s * 8, sda[0], sda[1], sda[2], sda[3]);
+          put4(FacL<3>::starA + s * 8 + 4, sda[4], sda[5], 0, 0);
+          for (int k = 4 * s; k < 12 * rm; k += 24) {
+            const double *p = srcA + e * 12 * rm + k;
+            put4(FacL<3>::src + k, p[0], p[1], p[2], p[3]);
+          }
         }
       }
     }

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(480, VGeo<T, O, R, RM>::ctasLift) kLiftVisc(co
     const FacU<T, O, R, RM> su{facPtr<T, O, R, RM>(a.fac, e), q};
 #pragma unroll
     for (int f = 0; f < 4; f++) su(f, ru.u[f]);
-    if (q < 12) liftRow<T, O, R>(a, a.face, wt, q, l, e, r, valid);
+    if (q < 12) liftRow<T, O, R, false>(a, a.face, wt, q, l, e, r, valid);
     cpAsyncWait<0>();
     __syncthreads();
     T acc[B];

@@ -330,8 +330,8 @@ int edge_b200_kernel_times(edge_b200_ctx *ctx, double *ms, int64_t *launches);
  * CTAs of the weak-form local / neighbour kernel. info[1], info[2] and info[5] describe the weak-form
  * kernels' buffers: info[1] 1 when face projections leave the local kernel pre-mixed with the reading
  * element's flux solver (per element face the padded pair [2][info[2]] of flux solvers in the
- * configuration's precision), 2 when there is also room for the characteristic rows through which
- * the LTS kernels mix, info[5] 1 when info[1] > 0 and fused steps are on. edge_b200_step_form tells
+ * configuration's precision), 2 when such a configuration's steps exchange characteristic rows (the
+ * strong form) as far as known, info[5] 1 when info[1] > 0 and fused steps are on. edge_b200_step_form tells
  * which form the GTS steps take. */
 int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]);
 /* The form of the context's next GTS step (EDGE_B200_EINVAL before mesh and element data are set):

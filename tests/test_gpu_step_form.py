@@ -71,3 +71,24 @@ def test_full_rank_flux_solvers_take_the_weak_form(order, runs, rm, prec):
     assert lib().edge_b200_upload_element_data(s._h, *ptrs) == 0
     assert lib().edge_b200_step_form(s._h) == 1
     s.close()
+
+
+@pytest.mark.parametrize("order,runs,prec", [(5, 16, 32), (3, 8, 32), (4, 1, 64)])
+def test_lts_in_strong_form_matches(order, runs, prec):
+    """Rate-2 LTS through the strong-form kernels (two-step sums, half-step rows, three groups)."""
+    import oracle
+    from test_lts import _grouped, _lts_state
+    prob, gf, flags, rel = _grouped(order=order, n=4, runs=runs, n_receivers=4, source="random", n_steps=30)
+    e0, _ = random_dofs(prob, seed=9, scale=1e-2)
+    ref = OracleRun(prob, e0.copy())
+    st = _lts_state(prob, e0.copy())
+    oracle.lts_cycles(ref.d, st, gf, 0.0, prob.dt, 2, flags, rel, ref.recv, ref.src)
+    s = Solver(prob, precision=prec)
+    assert lib().edge_b200_step_form(s._h) == 1
+    s.upload_dofs(e0.astype(s.dtype))
+    s.set_time_groups(gf)
+    s.step_lts(1)
+    s.step_lts(1)
+    e, _ = s.download_dofs()
+    assert rel_l2(e, st["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
+    s.close()
