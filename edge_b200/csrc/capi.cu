@@ -267,7 +267,8 @@ struct edge_b200_ctx {
   // sources
   SrcArgs src{};
   DevBuf srcMem[10];
-  DevBuf srcAmp;  // series integrals of the next steps (kSrcIntegrals)
+  DevBuf srcAmp;  // series integrals of the next steps (kSrcIntegrals): up to 1 MB of them, or one step's
+  int64_t srcAheadMax() const { return std::min<int64_t>(1024, std::max<int64_t>(1, 131072 / std::max(nSrc, 1))); }
   // per-source clocks and per-group time steps of merged simulations (edge_b200_set_source_clocks,
   // edge_b200_set_group_dt); srcStep counts the steps since the clocks were set
   DevBuf srcClk0, srcClkDt, grpDt;
@@ -527,6 +528,13 @@ struct edge_b200_ctx {
     stepRejected = nBad != 0;
     return cudaSuccess;
   }
+  // the same where the mesh and the element data are set: a step then finds them built (and a captured
+  // first step waits for nothing)
+  int buildStep() {
+    if (!meshSet || !dataSet) return EDGE_B200_OK;
+    cudaError_t e = ensureStep();
+    return e ? fail(e, "step coefficients") : EDGE_B200_OK;
+  }
   // what a GTS step of this context needs built
   cudaError_t ensureGts() {
     cudaError_t e = ensureStep();
@@ -537,6 +545,10 @@ struct edge_b200_ctx {
     stepRejected = false;
   }
 
+  int fail(cudaError_t e, const char *what) {
+    err = std::string(what) + ": " + cudaGetErrorString(e);
+    return EDGE_B200_EDEVICE;
+  }
   // after the stream was waited for: whether a part's rows arrived in the other form
   int checkHalo() {
     if (!haloBad.p) return EDGE_B200_OK;
@@ -548,10 +560,6 @@ struct edge_b200_ctx {
     return EDGE_B200_EMESH;
   }
 
-  int fail(cudaError_t e, const char *what) {
-    err = std::string(what) + ": " + cudaGetErrorString(e);
-    return EDGE_B200_EDEVICE;
-  }
   // weak: for the weak-form kernels (LTS), whatever form the GTS steps take
   StepArgsRaw args(double dt, bool weak = false) const {
     StepArgsRaw a;
@@ -698,7 +706,7 @@ int edge_b200_upload_mesh(edge_b200_ctx *ctx, const int32_t *el_fa_el, const uin
   ctx->hFaType.assign(el_fa_type, el_fa_type + n);
   ctx->meshSet = true;
   ctx->dataChanged();
-  return EDGE_B200_OK;
+  return ctx->buildStep();
 }
 
 int edge_b200_upload_element_data(edge_b200_ctx *ctx, const double *star_e, const double *fs_e,
@@ -724,7 +732,7 @@ int edge_b200_upload_element_data(edge_b200_ctx *ctx, const double *star_e, cons
   EDGE_CUDA(cudaStreamSynchronize(s), "upload element data");
   ctx->dataSet = true;
   ctx->dataChanged();
-  return EDGE_B200_OK;
+  return ctx->buildStep();
 }
 
 int edge_b200_share_element_data(edge_b200_ctx *dst, const edge_b200_ctx *src) {
@@ -746,7 +754,7 @@ int edge_b200_share_element_data(edge_b200_ctx *dst, const edge_b200_ctx *src) {
   ctx->sharedData = true;
   ctx->dataSet = true;
   ctx->dataChanged();
-  return EDGE_B200_OK;
+  return ctx->buildStep();
 }
 
 int edge_b200_upload_dofs(edge_b200_ctx *ctx, const void *dofs_e, const void *dofs_a) {
@@ -918,6 +926,7 @@ int edge_b200_set_sources(edge_b200_ctx *ctx, int n, const int64_t *el, const in
   ctx->src.ts = m[9].as<double>();
   ctx->src.tol = kTolTime;
   ctx->nSrc = n;
+  EDGE_CUDA(ctx->srcAmp.fit(size_t(ctx->srcAheadMax()) * n * sizeof(double)), "sources");
   EDGE_CUDA(cudaStreamSynchronize(s), "sources");
   return EDGE_B200_OK;
 }
@@ -1061,12 +1070,10 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
               "receiver schedule");
   }
   ctx->launches = 0;
-  // steps whose series integrals are computed together (one launch more, so not for a step or two),
-  // up to 1 MB of them at a time
+  // steps whose series integrals are computed together (one launch more, so not for a step or two)
   int srcAhead = 1;
   if (ctx->src.nGrp > 0 && ctx->rangeSrc && (phases & 1) && n_steps > 2) {
-    srcAhead = (int)std::min<int64_t>({int64_t(n_steps), 1024, std::max<int64_t>(1, 131072 / ctx->nSrc)});
-    EDGE_CUDA(ctx->srcAmp.fit(size_t(srcAhead) * ctx->nSrc * sizeof(double)), "source integrals");
+    srcAhead = (int)std::min<int64_t>(n_steps, ctx->srcAheadMax());
   }
   StepArgsRaw a = ctx->args(dt);
   if (ctx->rangeCount >= 0) {
