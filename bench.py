@@ -969,7 +969,10 @@ def main():
                 "batched_fp32_over_plain_fp64": value / (v64 * ws)}
         # the plain path against both ceilings: HBM (its algorithmic bytes per element) and the FP64
         # pipe (dense-equivalent flops over the nominal SMs x 64 FP64 FMA lanes x 2 x max SM clock)
-        alg64 = algorithmic(p64, 64)
+        strong64 = L.edge_b200_step_form(s64._h) == 1
+        alg64 = algorithmic(p64, 64, strong64)
+        if strong64:  # the step kernel is the whole step; the closing launch comes once per call
+            alg64["neigh_bytes"] = alg64["neigh_flops"] = 0
         sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         fp64_peak = sms * 64 * 2 * peak_clock_mhz() * 1e6 / 1e12
         tfl = (alg64["local_flops"] + alg64["neigh_flops"]) * v64 / 1e12
