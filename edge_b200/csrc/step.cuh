@@ -19,8 +19,9 @@
 //
 // Against the weak form with nine pre-mixed rows per face (one 9x9-rank mix for each side, a lift
 // for each side, volume product) this is 3,150 instead of 5,670 instructions per warp and element
-// group at order 5, nine barriers instead of thirteen, and 93 instead of 132 KB of device memory
-// traffic per element with 16 runs.
+// group at order 5, eight barriers instead of thirteen, and 90.5 KB of device memory traffic per element
+// with 16 runs. Whole steps, order 5: 663,552 elements, 16 runs, FP32 29.4 -> 18.3 ms; one run, FP64
+// 11.0 -> 3.98 ms. Bound: barriers and shared-memory latency at 18 warps per SM (issue 47%, DRAM 39%).
 #pragma once
 #include "kernels.cuh"
 
@@ -540,6 +541,7 @@ __device__ __forceinline__ void halfTask(const StepArgs<T> &a, const T *p, const
 // One GTS step of elements [elFirst, elFirst + elCount) up to their surface integrals: the pending
 // characteristics of the previous step (faceIn and wOwn, none when faceIn is null) complete the DOF
 // rows, the recursion updates them, and this step's characteristics leave in face and wOwn.
+// Measured (48,000 elements, order 5, 16 runs, FP32): 1.22 ms; order 4, 8 runs: 0.35 ms.
 // LTS 1, 2: the local step of a time group (rate-2 local time stepping; nothing is pending then): the
 // neighbours' rows also summed over two steps, and with 2 the half-step rows
 template <typename T, int O, int R, int LTS = 0>
@@ -730,7 +732,8 @@ __global__ void __launch_bounds__(SGeo<T, O, R>::NT, LTS == 2 ? 1 : SGeo<T, O, R
 }
 
 // The pending surface integrals on their own (the closing half of a step): face holds the
-// characteristics written for the elements by their neighbours, wOwn their own.
+// characteristics written for the elements by their neighbours, wOwn their own. Measured: 8.5 ms at
+// 663,552 elements, order 5, 16 runs, FP32 (4,963 GB/s of its bytes, 0.75 of the copy rate).
 template <typename T, int O, int R, bool LTS = false>
 __global__ void __launch_bounds__(SGeo<T, O, R>::NT, SGeo<T, O, R>::ctasLift) kLift(const StepArgs<T> a) {
   using G = SGeo<T, O, R>;
