@@ -540,9 +540,14 @@ struct edge_b200_ctx {
     cudaError_t e = ensureStep();
     return e || strong() ? e : ensureFsLR();
   }
+  // counts the changes of what a captured graph of this context's steps holds (a batch compares it
+  // with its value at the capture): element data and mesh, with them the step form and the buffers it
+  // writes, sources, clocks, time steps, element ranges, kept time integrals, launch shapes
+  int64_t stepGen = 0;
   void dataChanged() {
     fsLRStale = stepStale = true;
     stepRejected = false;
+    stepGen++;
   }
 
   int fail(cudaError_t e, const char *what) {
@@ -869,6 +874,7 @@ int edge_b200_keep_tdofs(edge_b200_ctx *ctx, int enable) {
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? EDGE_B200_ENOMEM : ctx->fail(e, "keep tDofs");
     EDGE_CUDA(cudaMemsetAsync(ctx->tDofs, 0, ctx->dofsCount() * ctx->realSize, ctx->stream), "keep tDofs");
   }
+  ctx->stepGen++;
   ctx->keepTDofs = enable != 0;
   return EDGE_B200_OK;
 }
@@ -884,6 +890,7 @@ int edge_b200_set_sources(edge_b200_ctx *ctx, int n, const int64_t *el, const in
                           const double *dt, const int64_t *ts_off, const int64_t *n_pts,
                           int64_t n_ts, const double *ts) {
   if (!ctx || n < 0) return EDGE_B200_EINVAL;
+  ctx->stepGen++;
   ctx->src = SrcArgs{};
   ctx->hSrcGrpEl.clear();
   ctx->nSrc = 0;
@@ -933,6 +940,7 @@ int edge_b200_set_sources(edge_b200_ctx *ctx, int n, const int64_t *el, const in
 
 int edge_b200_set_source_clocks(edge_b200_ctx *ctx, const double *t0, const double *dt) {
   if (!ctx) return EDGE_B200_EINVAL;
+  ctx->stepGen++;
   ctx->srcStep = 0;
   if (!t0 || !dt) {
     ctx->srcClocks = false;
@@ -953,12 +961,14 @@ int edge_b200_set_active_elements(edge_b200_ctx *ctx, int64_t n_active) {
   if (!ctx || n_active < 0 || n_active > ctx->nEl || ctx->nTg > 1) return EDGE_B200_EINVAL;
   // the pending neighbour step of a fused call covers the old range
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
+  ctx->stepGen++;
   ctx->nActive = n_active;
   return EDGE_B200_OK;
 }
 
 int edge_b200_set_group_dt(edge_b200_ctx *ctx, const double *dt_group) {
   if (!ctx) return EDGE_B200_EINVAL;
+  ctx->stepGen++;
   if (!dt_group) {
     ctx->grpDtOn = false;
     return EDGE_B200_OK;
@@ -1183,6 +1193,7 @@ int edge_b200_set_send_count(edge_b200_ctx *ctx, int64_t n_send) {
 int edge_b200_set_owned(edge_b200_ctx *ctx, int64_t n_owned) {
   if (!ctx || n_owned < 0 || n_owned > ctx->nEl || ctx->nTg > 1) return EDGE_B200_EINVAL;
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
+  ctx->stepGen++;
   ctx->nOwned = n_owned;
   return EDGE_B200_OK;
 }
@@ -1598,6 +1609,7 @@ struct edge_b200_batch {
   int32_t *activeDev = nullptr;
   cudaGraphExec_t exec = nullptr;  // two batch steps
   std::vector<char> fu;            // per context: fused steps, fixed when the graph is captured
+  std::vector<int64_t> gen;        // and its stepGen then (before the first capture: at creation)
   bool dirty = true;
   std::string err;
   ~edge_b200_batch() {
@@ -1675,7 +1687,10 @@ struct edge_b200_batch {
     if ((e = cudaStreamSynchronize(origin))) return e;
     // each context's step form for this graph and the direct launches around it
     fu.assign(ctxs.size(), 0);
-    for (size_t k = 0; k < ctxs.size(); k++) fu[k] = fused(ctxs[k]);
+    for (size_t k = 0; k < ctxs.size(); k++) {
+      fu[k] = fused(ctxs[k]);
+      if (active[k]) gen[k] = ctxs[k]->stepGen;
+    }
     if ((e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal))) return e;
     cudaError_t c = forkJoin([&](size_t k) {
       cudaError_t r = issueStep(k, 1, 0.0);
@@ -1700,10 +1715,11 @@ struct edge_b200_batch {
   // that nothing is pending when the call returns
   cudaError_t run(int n) {
     cudaError_t c;
-    // element data set since: coefficients again, and the graph with them
+    // contexts changed since the capture (new element data can change the step form, and with it what
+    // the steps' buffers hold): what their steps need built again, and the graph with it
     for (size_t k = 0; k < ctxs.size(); k++) {
       edge_b200_ctx *ctx = ctxs[k];
-      if (!active[k] || !ctx->stepStale || !ctx->ks->strongSupported()) continue;
+      if (!active[k] || gen[k] == ctx->stepGen) continue;
       if ((c = ctx->ensureGts()) || (c = cudaStreamSynchronize(ctx->stream))) return c;
       dirty = true;
     }
@@ -1777,6 +1793,7 @@ int edge_b200_batch_create(edge_b200_ctx *const *ctxs, int n, const double *t0, 
     edge_b200_ctx *c = ctxs[k];
     e = c->flush();
     if (!e) e = c->ensureGts();
+    b->gen.push_back(c->stepGen);
     if (!e) e = cudaEventRecord(b->joins[k], c->stream);
     if (!e) e = cudaStreamWaitEvent(b->origin, b->joins[k], 0);
   }
@@ -1876,6 +1893,7 @@ int edge_b200_autotune(edge_b200_ctx *ctx, double dt, int32_t caps[2]) {
   cudaEventDestroy(ev[0]);
   cudaEventDestroy(ev[1]);
   EDGE_CUDA(err, "autotune");
+  ctx->stepGen++;
   ks->setGridCaps(best[0], best[1]);
   EDGE_CUDA(cudaMemcpyAsync(ctx->dofsE, save.p, bytesE, cudaMemcpyDeviceToDevice, s), "autotune restore");
   if (bytesA)

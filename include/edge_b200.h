@@ -379,7 +379,9 @@ int edge_b200_step_noalloc(const edge_b200_cfg *cfg, int64_t n_el, double dt, in
  * graph is captured). Context k steps from time t0[k] by dt[k];
  * a device counter per context gives its sources the step's time. The contexts keep their data;
  * upload DOFs and element data before creating the batch, and call edge_b200_batch_sync before
- * using a context on its own again. Contexts with receivers, halo parts or kernel timing on are
+ * using a context on its own again. A context that gets another mesh, element data, sources, time
+ * steps or active range after such a sync takes them to the next batch step, which captures the graph
+ * again (and fixes its step form anew). Contexts with receivers, halo parts or kernel timing on are
  * refused (EDGE_B200_ENOTSUP): those run through edge_b200_step. No counterpart in the reference
  * (one solver per process; here uneven batches of simulations on one GPU). */
 typedef struct edge_b200_batch edge_b200_batch;

@@ -1,6 +1,8 @@
 """The strong-form GTS step is the one that runs: Godunov flux solvers of elastic and anelastic media
 are found to be of rank 3 (free surface, outflow, layered and jittered inner faces), other flux solvers
 send the context to the weak-form kernels, and both agree with the oracle."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -92,3 +94,74 @@ def test_lts_in_strong_form_matches(order, runs, prec):
     e, _ = s.download_dofs()
     assert rel_l2(e, st["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
     s.close()
+
+
+def _penalised(prob, share=0.05):
+    """A copy of the problem whose flux solvers penalise the jump at one inner face: full rank there."""
+    p = dataclasses.replace(prob, fsE=prob.fsE.copy())
+    e, f = map(int, np.argwhere(p.mesh.el_fa_type == 0)[5])
+    pen = share * np.abs(p.fsE[0, e, f].reshape(9, 9)).max(axis=1).min() * np.eye(9)
+    p.fsE[0, e, f] -= pen.ravel()
+    p.fsE[1, e, f] += pen.ravel()
+    return p
+
+
+def _upload_data(s, p):
+    arr = [None if v is None else np.ascontiguousarray(v, np.float64)
+           for v in (p.starE, p.fsE, p.starA, p.srcA, p.fsA, p.omega)]
+    assert lib().edge_b200_upload_element_data(s._h, *[None if v is None else v.ctypes.data for v in arr]) == 0
+
+
+@pytest.mark.parametrize("order,runs,rm,prec", [(5, 16, 0, 32), (4, 1, 0, 64), (5, 1, 0, 64), (4, 8, 3, 32)])
+def test_batch_takes_over_new_element_data(order, runs, rm, prec):
+    """Element data set between two calls of a batch: strong to strong with another material, strong to
+    weak, weak to weak, weak to strong and back; each call's result is the oracle's with the data of the
+    time."""
+    from edge_b200.batch import Batch
+    kw = dict(n=2, order=order, runs=runs, rm=rm, jitter=0.1, n_steps=3, source="random", n_receivers=0)
+    prob, layered = small_problem(**kw), small_problem(layers=[3000.0, 5000.0], **kw)
+    other = small_problem(n=2, order=3, runs=1, n_steps=3, source=None, n_receivers=0)
+    e0, a0 = random_dofs(prob, seed=2)
+    s, mate = Solver(prob, precision=prec), Solver(other, precision=64)
+    s.upload_dofs(e0, a0)
+    b = Batch([s, mate])
+    orc = OracleRun(prob, e0, a0)
+    for p, form in ((prob, 1), (layered, 1), (_penalised(prob), 0), (_penalised(layered), 0), (prob, 1),
+                    (_penalised(prob), 0)):
+        _upload_data(s, p)
+        assert lib().edge_b200_step_form(s._h) == form
+        b.run(4)
+        orc.d = p.oracle_dict()
+        orc.step(4)
+        got, _ = s.download_dofs()
+        assert rel_l2(got, orc.state["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
+    b.close()
+    s.close()
+    mate.close()
+
+
+def test_batch_takes_over_new_sources():
+    """A longer source list set between two calls of a batch (its arrays move)."""
+    from edge_b200.batch import Batch
+    prob = small_problem(n=2, order=4, runs=8, jitter=0.1, n_steps=12, source="random", n_receivers=0)
+    one = small_problem(n=2, order=4, runs=8, jitter=0.1, n_steps=12, source=None, n_receivers=0)
+    e0, _ = random_dofs(prob, seed=2, scale=1e-3)
+    s, ref = Solver(one, precision=32), Solver(one, precision=32)
+    src = prob.sources
+    from edge_b200._lib import ptr
+    b = Batch([s])
+    for x in (s, ref):
+        x.upload_dofs(e0)
+    b.run(3)
+    ref.step(3)
+    for x in (s, ref):
+        x._chk(lib().edge_b200_set_sources(x._h, src["n"], ptr(src["el"]), ptr(src["run"]), ptr(src["scal"]),
+                                           ptr(src["bEval"]), ptr(src["t0"]), ptr(src["dt"]), ptr(src["tsOff"]),
+                                           ptr(src["nPts"]), len(src["ts"]), ptr(src["ts"])), "set_sources")
+    b.run(6)
+    ref.step(6)
+    got, want = s.download_dofs()[0], ref.download_dofs()[0]
+    assert rel_l2(want, e0) > 1e-6 and rel_l2(got, want) < 1e-6
+    b.close()
+    s.close()
+    ref.close()
