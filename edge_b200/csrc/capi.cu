@@ -2,8 +2,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -221,6 +223,16 @@ static __global__ void kSrcIntegrals(SrcArgs s, int nSrc, int nSteps, double *ou
   }
 }
 
+// Element data on the device, held by the context that uploads them and by those that borrow them
+// (edge_b200_share_element_data), freed with the last. gen counts the uploads: what a borrower derived
+// from the arrays (its step coefficients, flux-solver pairs) is built again when it has moved.
+struct ElementData {
+  double *starE = nullptr, *starA = nullptr, *srcA = nullptr, *fsE = nullptr, *fsA = nullptr;
+  double omega[3] = {0, 0, 0};
+  std::atomic<int64_t> gen{0};
+  ~ElementData() { dfree(starE); dfree(starA); dfree(srcA); dfree(fsE); dfree(fsA); }
+};
+
 struct edge_b200_ctx {
   edge_b200_cfg cfg{};
   int64_t nEl = 0;
@@ -237,10 +249,11 @@ struct edge_b200_ctx {
   KernelSet *ks = nullptr;
   // resident device data
   void *dofsE = nullptr, *dofsA = nullptr, *tDofs = nullptr, *face = nullptr;
-  double *starE = nullptr, *starA = nullptr, *srcA = nullptr, *fsE = nullptr, *fsA = nullptr;
+  std::shared_ptr<ElementData> data = std::make_shared<ElementData>();
+  bool borrowed = false;  // data belong to another context
+  int64_t dataGen = 0;    // data->gen of what was built from them
   int32_t *elFaEl = nullptr;
   uint8_t *fId = nullptr, *vId = nullptr, *faType = nullptr;
-  double omega[3] = {0, 0, 0};
   bool meshSet = false, dataSet = false, keepTDofs = false;
   // flux-solver pairs of the pre-mixed face projections (configurations with KernelSet::premix),
   // rebuilt before the next GTS step after the mesh or the element data changed
@@ -485,6 +498,7 @@ struct edge_b200_ctx {
 
   // the flux-solver pairs of the pre-mixed projections (weak form)
   cudaError_t ensureFsLR() {
+    refreshData();
     if (!ks->premix() || !fsLRStale) return cudaSuccess;
     const int P = ks->fsPairStride();
     cudaError_t e = fsLR.fit(size_t(nEl) * 4 * 2 * P * realSize);
@@ -492,9 +506,9 @@ struct edge_b200_ctx {
     const int64_t total = nEl * 4 * 2 * P;
     const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
     if (cfg.precision == 64)
-      kBuildFsLR<double><<<grid, 256, 0, stream>>>(fsE, elFaEl, fId, faType, nEl, P, fsLR.as<double>());
+      kBuildFsLR<double><<<grid, 256, 0, stream>>>(data->fsE, elFaEl, fId, faType, nEl, P, fsLR.as<double>());
     else
-      kBuildFsLR<float><<<grid, 256, 0, stream>>>(fsE, elFaEl, fId, faType, nEl, P, fsLR.as<float>());
+      kBuildFsLR<float><<<grid, 256, 0, stream>>>(data->fsE, elFaEl, fId, faType, nEl, P, fsLR.as<float>());
     if ((e = cudaGetLastError())) return e;
     fsLRStale = false;
     return cudaSuccess;
@@ -502,6 +516,7 @@ struct edge_b200_ctx {
 
   // the coefficients of the strong-form step, for configurations that have it
   cudaError_t ensureStep() {
+    refreshData();
     if (!ks->strongSupported() || !stepStale || stepRejected) return cudaSuccess;
     if (nEl >= (int64_t(1) << 28)) {  // beyond the packed gather table
       stepRejected = true;
@@ -515,12 +530,13 @@ struct edge_b200_ctx {
     if ((e = cudaMemsetAsync(bad, 0, sizeof(int), stream))) return e;
     const int64_t work = (nEl * 4 + kTeams * kBuildWarps - 1) / (kTeams * kBuildWarps);
     const int grid = (int)std::min<int64_t>(work, 148 * 32);
+    const ElementData &d = *data;
     if (cfg.precision == 64)
-      kBuildStep<double><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
-                                                  static_cast<double *>(fac), gath, bad);
+      kBuildStep<double><<<grid, kBuildWarps * 32, 0, stream>>>(d.fsE, d.starE, d.fsA, d.starA, d.srcA, cfg.n_rms, elFaEl, fId, vId,
+                                                              faType, nEl, cfg.order, E, static_cast<double *>(fac), gath, bad);
     else
-      kBuildStep<float><<<grid, kBuildWarps * 32, 0, stream>>>(fsE, starE, fsA, starA, srcA, cfg.n_rms, elFaEl, fId, vId, faType, nEl, cfg.order, E,
-                                                 static_cast<float *>(fac), gath, bad);
+      kBuildStep<float><<<grid, kBuildWarps * 32, 0, stream>>>(d.fsE, d.starE, d.fsA, d.starA, d.srcA, cfg.n_rms, elFaEl, fId, vId,
+                                                              faType, nEl, cfg.order, E, static_cast<float *>(fac), gath, bad);
     if ((e = cudaGetLastError())) return e;
     if ((e = cudaMemcpyAsync(&nBad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream))) return e;
     if ((e = cudaStreamSynchronize(stream))) return e;
@@ -548,6 +564,11 @@ struct edge_b200_ctx {
     fsLRStale = stepStale = true;
     stepRejected = false;
     stepGen++;
+    dataGen = data->gen;
+  }
+  // new data in the arrays this context borrows
+  void refreshData() {
+    if (data->gen != dataGen) dataChanged();
   }
 
   int fail(cudaError_t e, const char *what) {
@@ -579,11 +600,11 @@ struct edge_b200_ctx {
     } else {
       a.face = face;
     }
-    a.starE = starE;
-    a.starA = starA;
-    a.srcA = srcA;
-    a.fsE = fsE;
-    a.fsA = fsA;
+    a.starE = data->starE;
+    a.starA = data->starA;
+    a.srcA = data->srcA;
+    a.fsE = data->fsE;
+    a.fsA = data->fsA;
     a.elFaEl = elFaEl;
     a.fId = fId;
     a.vId = vId;
@@ -594,16 +615,11 @@ struct edge_b200_ctx {
     a.elFirst = 0;
     a.elCount = std::min(nOwned, nActive);
     a.dt = dt;
-    for (int i = 0; i < 3; i++) a.omega[i] = omega[i];
+    for (int i = 0; i < 3; i++) a.omega[i] = data->omega[i];
     return a;
   }
-  // element data borrowed from another context (edge_b200_share_element_data): not freed here
-  bool sharedData = false;
   ~edge_b200_ctx() {
     dfree(dofsE); dfree(dofsA); dfree(tDofs); dfree(face);
-    if (!sharedData) {
-      dfree(starE); dfree(starA); dfree(srcA); dfree(fsE); dfree(fsA);
-    }
     dfree(elFaEl); dfree(fId); dfree(vId); dfree(faType);
     dfree(dTau); dfree(dSlot); dfree(stage);
     for (int i = 0; i < kSlots; i++) dfree(slotIn[i]);
@@ -722,19 +738,21 @@ int edge_b200_upload_element_data(edge_b200_ctx *ctx, const double *star_e, cons
   if (rm && (!star_a || !src_a || !fs_a || !omega)) return EDGE_B200_EINVAL;
   cudaStream_t s = ctx->stream;
   const size_t n = ctx->nEl;
-  if (ctx->sharedData) {  // stop borrowing: this context gets arrays of its own
-    ctx->starE = ctx->starA = ctx->srcA = ctx->fsE = ctx->fsA = nullptr;
-    ctx->sharedData = false;
+  if (ctx->borrowed) {  // stop borrowing: this context gets arrays of its own
+    ctx->data = std::make_shared<ElementData>();
+    ctx->borrowed = false;
   }
-  EDGE_CUDA(upload(ctx->starE, star_e, n * 72 * sizeof(double), s), "upload starE");
-  EDGE_CUDA(upload(ctx->fsE, fs_e, n * 2 * 4 * 81 * sizeof(double), s), "upload fsE");
+  ElementData &d = *ctx->data;
+  EDGE_CUDA(upload(d.starE, star_e, n * 72 * sizeof(double), s), "upload starE");
+  EDGE_CUDA(upload(d.fsE, fs_e, n * 2 * 4 * 81 * sizeof(double), s), "upload fsE");
   if (rm) {
-    EDGE_CUDA(upload(ctx->starA, star_a, n * 27 * sizeof(double), s), "upload starA");
-    EDGE_CUDA(upload(ctx->srcA, src_a, n * rm * 12 * sizeof(double), s), "upload srcA");
-    EDGE_CUDA(upload(ctx->fsA, fs_a, n * 2 * 4 * 54 * sizeof(double), s), "upload fsA");
-    for (int m = 0; m < rm; m++) ctx->omega[m] = omega[m];
+    EDGE_CUDA(upload(d.starA, star_a, n * 27 * sizeof(double), s), "upload starA");
+    EDGE_CUDA(upload(d.srcA, src_a, n * rm * 12 * sizeof(double), s), "upload srcA");
+    EDGE_CUDA(upload(d.fsA, fs_a, n * 2 * 4 * 54 * sizeof(double), s), "upload fsA");
+    for (int m = 0; m < rm; m++) d.omega[m] = omega[m];
   }
   EDGE_CUDA(cudaStreamSynchronize(s), "upload element data");
+  d.gen++;
   ctx->dataSet = true;
   ctx->dataChanged();
   return ctx->buildStep();
@@ -747,16 +765,8 @@ int edge_b200_share_element_data(edge_b200_ctx *dst, const edge_b200_ctx *src) {
   edge_b200_ctx *ctx = dst;
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
   EDGE_CUDA(cudaStreamSynchronize(ctx->stream), "share element data");
-  if (!ctx->sharedData) {
-    dfree(ctx->starE); dfree(ctx->starA); dfree(ctx->srcA); dfree(ctx->fsE); dfree(ctx->fsA);
-  }
-  ctx->starE = src->starE;
-  ctx->starA = src->starA;
-  ctx->srcA = src->srcA;
-  ctx->fsE = src->fsE;
-  ctx->fsA = src->fsA;
-  for (int m = 0; m < 3; m++) ctx->omega[m] = src->omega[m];
-  ctx->sharedData = true;
+  ctx->data = src->data;
+  ctx->borrowed = true;
   ctx->dataSet = true;
   ctx->dataChanged();
   return ctx->buildStep();
@@ -1719,6 +1729,7 @@ struct edge_b200_batch {
     // the steps' buffers hold): what their steps need built again, and the graph with it
     for (size_t k = 0; k < ctxs.size(); k++) {
       edge_b200_ctx *ctx = ctxs[k];
+      ctx->refreshData();
       if (!active[k] || gen[k] == ctx->stepGen) continue;
       if ((c = ctx->ensureGts()) || (c = cudaStreamSynchronize(ctx->stream))) return c;
       dirty = true;

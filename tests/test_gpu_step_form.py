@@ -96,13 +96,13 @@ def test_lts_in_strong_form_matches(order, runs, prec):
     s.close()
 
 
-def _penalised(prob, share=0.05):
-    """A copy of the problem whose flux solvers penalise the jump at one inner face: full rank there."""
+def _penalised(prob, share=0.05, faces=slice(5, 6)):
+    """A copy of the problem whose flux solvers penalise the jump at some inner faces: full rank there."""
     p = dataclasses.replace(prob, fsE=prob.fsE.copy())
-    e, f = map(int, np.argwhere(p.mesh.el_fa_type == 0)[5])
-    pen = share * np.abs(p.fsE[0, e, f].reshape(9, 9)).max(axis=1).min() * np.eye(9)
-    p.fsE[0, e, f] -= pen.ravel()
-    p.fsE[1, e, f] += pen.ravel()
+    for e, f in np.argwhere(p.mesh.el_fa_type == 0)[faces]:
+        pen = share * np.abs(p.fsE[0, e, f].reshape(9, 9)).max(axis=1).min() * np.eye(9)
+        p.fsE[0, e, f] -= pen.ravel()
+        p.fsE[1, e, f] += pen.ravel()
     return p
 
 
@@ -165,3 +165,39 @@ def test_batch_takes_over_new_sources():
     b.close()
     s.close()
     ref.close()
+
+
+@pytest.mark.parametrize("order,runs,rm,prec", [(5, 16, 0, 32), (4, 1, 0, 64), (5, 1, 0, 64), (4, 8, 3, 32), (6, 4, 3, 32)])
+def test_borrowers_follow_new_element_data(order, runs, rm, prec):
+    """A context that borrows element data steps (and samples its receivers) with what its lender
+    uploads later, in the form that those data allow, on its own and in a batch."""
+    from edge_b200.batch import Batch
+    kw = dict(n=2, order=order, runs=runs, rm=rm, jitter=0.1, n_steps=12, source=None)
+    prob, layered = small_problem(**kw), small_problem(layers=[3000.0, 5000.0], **kw)
+    e0, a0 = random_dofs(prob, seed=6)
+    lender = Solver(prob, precision=prec)
+    s = Solver(prob, precision=prec, share_from=lender)
+    quiet = Solver(dataclasses.replace(prob, receivers=None), precision=prec, share_from=s)  # borrows through s
+    b = Batch([quiet])
+    s.upload_dofs(e0, a0)
+    quiet.upload_dofs(e0, a0)
+    orc = OracleRun(prob, e0, a0)
+    tol = 1e-12 if prec == 64 else 1e-4
+    strong = lib().edge_b200_step_form(lender._h)
+    for p, form in ((prob, strong), (layered, strong), (_penalised(layered), 0), (prob, strong)):
+        for x in (s, quiet):
+            x.sync()
+        _upload_data(lender, p)
+        s.step(3)
+        b.run(3)
+        assert lib().edge_b200_step_form(s._h) == form
+        orc.d = p.oracle_dict()
+        orc.step(3)
+        for x in (s, quiet):
+            assert rel_l2(x.download_dofs()[0], orc.state["dofsE"]) < tol
+    rb, _, rc = s.receivers()
+    k = int(rc[0])
+    assert k > 0 and rel_l2(rb[:, :k], orc.recv["buf"][:, :k]) < tol
+    b.close()
+    for x in (lender, quiet, s):  # the lender first: the data live as long as a borrower
+        x.close()
