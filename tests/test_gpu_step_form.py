@@ -201,3 +201,40 @@ def test_borrowers_follow_new_element_data(order, runs, rm, prec):
     b.close()
     for x in (lender, quiet, s):  # the lender first: the data live as long as a borrower
         x.close()
+
+
+@pytest.mark.parametrize("order,rm", [(4, 0), (5, 0), (4, 3)])
+@pytest.mark.parametrize("share", [3e-9, 1e-10, 3e-12])
+def test_small_full_rank_parts_are_kept_in_fp64(order, rm, share):
+    """Flux solvers a little off rank 3 at every inner face: what they add to the result (seen against
+    the oracle with and without it) is not dropped."""
+    prob = small_problem(n=2, order=order, runs=1, rm=rm, jitter=0.1, n_steps=3, source=None, n_receivers=0)
+    off = _penalised(prob, share, slice(None))
+    e0, a0 = random_dofs(prob, seed=8)
+    e0[:, 6:] *= 1e-7  # velocities of the stresses' energy: both rows of a solver count
+    s = Solver(off, precision=64)
+    s.upload_dofs(e0, a0)
+    s.step(4)
+    orc, plain = (OracleRun(p, e0.copy(), None if a0 is None else a0.copy()) for p in (off, prob))
+    orc.step(4)
+    plain.step(4)
+    got, _ = s.download_dofs()
+    for q in (slice(0, 6), slice(6, 9)):
+        added = rel_l2(plain.state["dofsE"][:, q], orc.state["dofsE"][:, q])
+        assert rel_l2(got[:, q], orc.state["dofsE"][:, q]) < 0.1 * added + 1e-14
+    s.close()
+
+
+@pytest.mark.parametrize("order,rm", [(4, 0), (4, 3)])
+def test_godunov_solvers_of_strong_contrasts_take_the_strong_form(order, rm):
+    prob = small_problem(n=4, order=order, runs=1, rm=rm, jitter=0.2, n_steps=3, layers=[300.0, 9000.0],
+                         lognormal_sigma=1.0, n_receivers=0)
+    e0, a0 = random_dofs(prob, seed=8)
+    s = Solver(prob, precision=64)
+    assert lib().edge_b200_step_form(s._h) == 1
+    s.upload_dofs(e0, a0)
+    s.step(4)
+    orc = OracleRun(prob, e0, a0)
+    orc.step(4)
+    assert rel_l2(s.download_dofs()[0], orc.state["dofsE"]) < 1e-12
+    s.close()
