@@ -11,10 +11,10 @@
 #include <vector>
 
 #include "../../include/edge_b200.h"
+#include "halo.cuh"
 #include "kernel_set.h"
 #include "kernels.cuh"
 #include "layout.cuh"
-#include "step_coef.cuh"
 
 namespace edge_b200 {
 KernelSet *makeKernelSet_o2(int, int, int, int);
@@ -95,33 +95,6 @@ __global__ void kBuildFsLR(const double *fsE, const int32_t *elFaEl, const uint8
       }
     }
     out[i] = T(v);
-  }
-}
-
-// halo exchange: the rows of face slots (element * 4 + face) to / from a packed buffer with stride16 x
-// 16 bytes per slot, 16 bytes per thread; slots outside the face buffer are skipped. Weak form: nine
-// pre-mixed rows; strong form: three characteristic rows and a mark behind them, by which a part
-// notices rows of the other form (*bad counts them; they are not taken over).
-constexpr uint4 kHaloMark = {0x7fa5c3e1u, 0x51e0c4a7u, 0x7fe1a5c3u, 0x0c4a751eu};
-__global__ void kFacePack(uint4 *face, uint4 *buf, const int32_t *slots, int n, int64_t stride16, int64_t nSlots,
-                          bool strong, bool pack, int *bad) {
-  const int64_t blk16 = strong ? stride16 / 3 : stride16, total = (int64_t)n * blk16;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t k = i / blk16, w = i % blk16;
-    const int64_t sl = slots[k];
-    if (sl < 0 || sl >= nSlots) continue;
-    uint4 *mark = buf + k * stride16 + stride16 / 3;
-    if (pack) {
-      buf[k * stride16 + w] = face[sl * blk16 + w];
-      if (strong && w == 0) *mark = kHaloMark;
-      continue;
-    }
-    const uint4 m = *mark;
-    const bool isStrong = m.x == kHaloMark.x && m.y == kHaloMark.y && m.z == kHaloMark.z && m.w == kHaloMark.w;
-    if (isStrong == strong)
-      face[sl * blk16 + w] = buf[k * stride16 + w];
-    else if (w == 0)
-      atomicAdd(bad, 1);
   }
 }
 
@@ -276,7 +249,9 @@ struct edge_b200_ctx {
   bool pending = false, fusedOn = true;
   char *faceThird(int i) const { return static_cast<char *>(face) + i * (faceCount() / 3 * realSize); }
   void *outBuf(int i) const { return faceThird(i); }
-  DevBuf haloBad;  // blocks unpacked in the other form (kFacePack)
+  // the face that reads each face slot: parts turn halo rows of the other form (kFaceUnpack)
+  DevBuf readers;
+  bool readersStale = true;
   // sources
   SrcArgs src{};
   DevBuf srcMem[10];
@@ -544,6 +519,17 @@ struct edge_b200_ctx {
     stepRejected = nBad != 0;
     return cudaSuccess;
   }
+  cudaError_t ensureReaders() {
+    if (!meshSet || !ks->strongSupported() || !readersStale) return cudaSuccess;
+    cudaError_t e;
+    if ((e = readers.fit(size_t(nEl) * 4 * sizeof(uint32_t)))) return e;
+    if ((e = cudaMemsetAsync(readers.p, 0xff, size_t(nEl) * 4 * sizeof(uint32_t), stream))) return e;
+    kFaceReaders<<<(int)std::min<int64_t>((nEl * 4 + 255) / 256, 148 * 16), 256, 0, stream>>>(
+        elFaEl, fId, faType, nEl * 4, readers.as<uint32_t>());
+    if ((e = cudaGetLastError())) return e;
+    readersStale = false;
+    return cudaSuccess;
+  }
   // the same where the mesh and the element data are set: a step then finds them built (and a captured
   // first step waits for nothing)
   int buildStep() {
@@ -575,17 +561,6 @@ struct edge_b200_ctx {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return EDGE_B200_EDEVICE;
   }
-  // after the stream was waited for: whether a part's rows arrived in the other form
-  int checkHalo() {
-    if (!haloBad.p) return EDGE_B200_OK;
-    int n = 0;
-    cudaError_t e = cudaMemcpy(&n, haloBad.p, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e) return fail(e, "halo check");
-    if (n == 0) return EDGE_B200_OK;
-    err = "halo rows of the other step form arrived: the flux solvers of only some parts have rank 3";
-    return EDGE_B200_EMESH;
-  }
-
   // weak: for the weak-form kernels (LTS), whatever form the GTS steps take
   StepArgsRaw args(double dt, bool weak = false) const {
     StepArgsRaw a;
@@ -727,6 +702,8 @@ int edge_b200_upload_mesh(edge_b200_ctx *ctx, const int32_t *el_fa_el, const uin
   ctx->hFaType.assign(el_fa_type, el_fa_type + n);
   ctx->meshSet = true;
   ctx->dataChanged();
+  ctx->readersStale = true;
+  if (ctx->nOwned < ctx->nEl) EDGE_CUDA(ctx->ensureReaders(), "face readers");
   return ctx->buildStep();
 }
 
@@ -785,7 +762,7 @@ int edge_b200_download_dofs(edge_b200_ctx *ctx, void *dofs_e, void *dofs_a) {
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
   EDGE_CUDA(ctx->downloadRows(dofs_e, ctx->dofsE, 9), "download dofsE");
   if (ctx->cfg.n_rms && dofs_a) EDGE_CUDA(ctx->downloadRows(dofs_a, ctx->dofsA, 6 * ctx->cfg.n_rms), "download dofsA");
-  return ctx->checkHalo();
+  return EDGE_B200_OK;
 }
 
 int edge_b200_upload_dofs_async(edge_b200_ctx *ctx, const void *dofs_e, const void *dofs_a) {
@@ -1205,6 +1182,7 @@ int edge_b200_set_owned(edge_b200_ctx *ctx, int64_t n_owned) {
   EDGE_CUDA(ctx->flush(), "pending neighbour step");
   ctx->stepGen++;
   ctx->nOwned = n_owned;
+  if (n_owned < ctx->nEl) EDGE_CUDA(ctx->ensureReaders(), "face readers");
   return EDGE_B200_OK;
 }
 
@@ -1216,17 +1194,24 @@ static int packFaces(edge_b200_ctx *ctx, int n, const int32_t *slots, void *buf,
   if (!ctx || n < 0 || (n && (!slots || !buf))) return EDGE_B200_EINVAL;
   if (n == 0) return EDGE_B200_OK;
   if (ctx->meshSet && ctx->dataSet) EDGE_CUDA(ctx->ensureGts(), "step coefficients");
-  if (!ctx->haloBad.p) {
-    EDGE_CUDA(ctx->haloBad.fit(sizeof(int)), "halo check");
-    EDGE_CUDA(cudaMemsetAsync(ctx->haloBad.p, 0, sizeof(int), ctx->stream), "halo check");
-  }
   const bool st = ctx->strong();
-  const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16;
-  const int64_t total = (int64_t)n * (st ? stride16 / 3 : stride16);
-  const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
-  kFacePack<<<grid, 256, 0, ctx->stream>>>(static_cast<uint4 *>(st ? ctx->outBuf(ctx->outCur) : ctx->face),
-                                           static_cast<uint4 *>(buf), slots, n, stride16, ctx->nEl * 4, st, pack,
-                                           ctx->haloBad.as<int>());
+  const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16, nSlots = ctx->nEl * 4;
+  uint4 *face = static_cast<uint4 *>(st ? ctx->outBuf(ctx->outCur) : ctx->face), *blocks = static_cast<uint4 *>(buf);
+  cudaStream_t s = ctx->stream;
+  if (pack) {
+    const int64_t total = (int64_t)n * (st ? stride16 / 3 : stride16);
+    kFacePack<<<(int)std::min<int64_t>((total + 255) / 256, 148 * 16), 256, 0, s>>>(face, blocks, slots, n, stride16,
+                                                                                   nSlots, st);
+  } else {
+    EDGE_CUDA(ctx->ensureReaders(), "face readers");
+    const uint32_t *reader = ctx->dataSet && !ctx->readersStale ? ctx->readers.as<uint32_t>() : nullptr;
+    const int grid = (int)std::min<int64_t>((n + kBuildWarps - 1) / kBuildWarps, 148 * 16);
+    const auto unpack = [&](auto kernel) {
+      kernel<<<grid, kBuildWarps * 32, 0, s>>>(face, blocks, slots, n, stride16, nSlots, ctx->cfg.n_runs, st,
+                                               ctx->ks->premix(), ctx->data->fsE, reader);
+    };
+    ctx->cfg.precision == 64 ? unpack(kFaceUnpack<double>) : unpack(kFaceUnpack<float>);
+  }
   EDGE_CUDA(cudaGetLastError(), pack ? "pack faces" : "unpack faces");
   return EDGE_B200_OK;
 }
@@ -1540,7 +1525,7 @@ int edge_b200_sync(edge_b200_ctx *ctx) {
   if (ctx->h2d) EDGE_CUDA(cudaStreamSynchronize(ctx->h2d), "sync");
   if (ctx->d2h) EDGE_CUDA(cudaStreamSynchronize(ctx->d2h), "sync");
   EDGE_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-  return ctx->checkHalo();
+  return EDGE_B200_OK;
 }
 
 int edge_b200_device_dofs(edge_b200_ctx *ctx, void **dofs_e, void **dofs_a, void **tdofs) {

@@ -116,6 +116,47 @@ __device__ __forceinline__ double rowBasis(FaceTeam &t, int a, double (&S)[9], d
   return res;
 }
 
+// U = A^T R of the team's U (9 x 3): three orthonormal columns A and the triangle R; a column without
+// anything left is zero
+__device__ __forceinline__ void qrU(const FaceTeam &t, double (&A)[3][9], double (&Rm)[3][3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double v[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) v[i] = t.U[i][k];
+#pragma unroll
+    for (int kk = 0; kk < 3; kk++) Rm[kk][k] = 0;
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+      for (int kk = 0; kk < k; kk++) {
+        double d = 0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) d += v[i] * A[kk][i];
+        Rm[kk][k] += d;
+#pragma unroll
+        for (int i = 0; i < 9; i++) v[i] -= d * A[kk][i];
+      }
+    double l2 = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) l2 += v[i] * v[i];
+    const double len = sqrt(l2), inv = len > 1e-12 ? 1.0 / len : 0.0;
+    Rm[k][k] = len > 1e-12 ? len : 0.0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) A[k][i] = v[i] * inv;
+  }
+}
+// R x = b
+__device__ __forceinline__ void solveR(const double (&Rm)[3][3], const double (&b)[3], double (&x)[3]) {
+#pragma unroll
+  for (int k = 2; k >= 0; k--) {
+    double v = b[k];
+#pragma unroll
+    for (int kk = k + 1; kk < 3; kk++) v -= Rm[k][kk] * x[kk];
+    x[k] = Rm[k][k] > 0 ? v / Rm[k][k] : 0.0;
+  }
+}
+
 // Per face: V1 of its reader (a function of the reader's fsE[1] alone, so that parts of a partition agree
 // on it), U and V0; with face 0 the element's other coefficients. Counts lanes that find solvers not of
 // rank 3 in this form in *bad. Values leave as whole 16-byte chunks.
@@ -239,32 +280,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
     for (int j = 0; j < 9; j++) t.N[a][j] = N[j] / sc.r(a);
     __syncwarp();
     double A[3][9], Rm[3][3], b[3], x[3], nj[9];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      double v[9];
-#pragma unroll
-      for (int i2 = 0; i2 < 9; i2++) v[i2] = t.U[i2][k];
-#pragma unroll
-      for (int kk = 0; kk < 3; kk++) Rm[kk][k] = 0;
-#pragma unroll
-      for (int pass = 0; pass < 2; pass++)
-#pragma unroll
-        for (int kk = 0; kk < k; kk++) {
-          double d = 0;
-#pragma unroll
-          for (int i2 = 0; i2 < 9; i2++) d += v[i2] * A[kk][i2];
-          Rm[kk][k] += d;
-#pragma unroll
-          for (int i2 = 0; i2 < 9; i2++) v[i2] -= d * A[kk][i2];
-        }
-      double l2 = 0;
-#pragma unroll
-      for (int i2 = 0; i2 < 9; i2++) l2 += v[i2] * v[i2];
-      const double len2 = sqrt(l2), inv = len2 > 1e-12 ? 1.0 / len2 : 0.0;
-      Rm[k][k] = len2 > 1e-12 ? len2 : 0.0;
-#pragma unroll
-      for (int i2 = 0; i2 < 9; i2++) A[k][i2] = v[i2] * inv;
-    }
+    qrU(t, A, Rm);
 #pragma unroll
     for (int i2 = 0; i2 < 9; i2++) nj[i2] = t.N[i2][a];
     double res = 0;
@@ -279,13 +295,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32)
       const double d = nj[i2] - A[0][i2] * b[0] - A[1][i2] * b[1] - A[2][i2] * b[2];
       res += d * d;
     }
-#pragma unroll
-    for (int k = 2; k >= 0; k--) {
-      double v = b[k];
-#pragma unroll
-      for (int kk = k + 1; kk < 3; kk++) v -= Rm[k][kk] * x[kk];
-      x[k] = Rm[k][k] > 0 ? v / Rm[k][k] : 0.0;
-    }
+    solveR(Rm, b, x);
 #pragma unroll
     for (int k = 0; k < 3; k++) t.V0[a][k] = x[k];
     put4(V + 8 * a, x[0], x[1], x[2], v1[0]);

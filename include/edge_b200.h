@@ -266,10 +266,9 @@ int edge_b200_wavefield(edge_b200_ctx *ctx, float *out);
  * [9][R][GF] of n face slots (slots[i] = element * 4 + face, a device int32 array) to / from the
  * device buffer out / in ([n] blocks of edge_b200_face_block_bytes each, GF = F rounded up to 16
  * bytes; in the strong form a block holds the three characteristic rows of its face), ordered on the
- * context stream; slots outside the mesh are skipped. All parts have to take the same form
- * (edge_b200_step_form): rows of the other one are not taken over, and edge_b200_sync and
- * edge_b200_download_dofs then return EDGE_B200_EMESH. Time groups need the
- * whole mesh owned. To overlap the exchange with work, as the reference's inner / send regions do
+ * context stream; slots outside the mesh are skipped. Parts may take different forms
+ * (edge_b200_step_form): unpack turns rows of the other one into its own. Time groups need the whole
+ * mesh owned. To overlap the exchange with work, as the reference's inner / send regions do
  * (src/impl/seismic/setup.inc:337-399), number the owned elements with a face neighbour in another
  * part first and give their count to edge_b200_set_send_count: phase 2 runs the receivers and the
  * local step of those [0, n_send), phase 3 the local step of the others [n_send, n_owned) and the

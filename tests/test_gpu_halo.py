@@ -86,3 +86,67 @@ def test_send_then_inner_equals_whole_local_step():
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][2], out[1][2]) and int(out[0][2][0]) > 0
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n_parts,precision,order,runs,rm", [(2, 64, 4, 1, 0), (2, 64, 5, 1, 0), (3, 32, 5, 16, 0),
+                                                             (2, 32, 6, 4, 0), (2, 32, 4, 8, 3), (2, 64, 4, 1, 3)])
+def test_parts_of_different_forms(n_parts, precision, order, runs, rm):
+    """One part's flux solvers are full rank at one face, so it takes the weak form and the others the
+    strong one (pre-mixed rows or projections against characteristics): the parts still equal the
+    oracle's one domain; with Godunov solvers again in every part, they do in one form."""
+    from edge_b200._lib import lib, ptr
+    from helpers import OracleRun
+    prob = host.build_problem(4, order, runs, rm=rm, jitter=0.15, seed=12, n_receivers=0, source=None,
+                              layers=[3000.0, 5000.0])
+    good = prob.fsE.copy()
+    plan = shard.plan(prob.mesh, n_parts)
+    p = plan[n_parts // 2]
+    far = p.owned[p.n_send:]  # no other part knows these elements
+    e, f = next((e, f) for e in far for f in range(4)
+                if prob.mesh.el_fa_type[e, f] == host.FACE_INNER and prob.mesh.el_fa_el[e, f] in far)
+    pen = 0.05 * np.abs(prob.fsE[0, e, f].reshape(9, 9)).max(axis=1).min() * np.eye(9)
+    prob.fsE[0, e, f] -= pen.ravel()
+    prob.fsE[1, e, f] += pen.ravel()
+    e0, a0 = random_dofs(prob, seed=5, scale=1e-2)
+    orc = OracleRun(prob, e0.copy(), None if a0 is None else a0.copy())
+    parts = [shard.PartSolver(prob, q, precision=precision) for q in plan]
+    tol = 1e-12 if precision == 64 else 1e-4
+
+    def steps(n, t):
+        for _ in range(n):
+            for ps in parts:
+                ps.phase0(t, prob.dt)
+            sent = {ps.part.rank: ps.pack() for ps in parts}
+            for ps in parts:
+                for q, buf in ps.recv_buf.items():
+                    buf.copy_(sent[q][ps.part.rank])
+                ps.unpack()
+            for ps in parts:
+                ps.phase1(t, prob.dt)
+            t += prob.dt
+        for k in range(2 if rm else 1):
+            got = np.concatenate([ps.download_owned()[k] for ps in parts])
+            assert rel_l2(got, orc.state["dofsA" if k else "dofsE"]) < tol
+        return t
+
+    try:
+        for ps in parts:
+            ids = ps.part.global_ids()
+            ps.solver.upload_dofs(e0[ids], None if a0 is None else a0[ids])
+        forms = [lib().edge_b200_step_form(ps.solver._h) for ps in parts]
+        assert forms == [0 if q is p else 1 for q in plan]
+        orc.step(5)
+        t = steps(5, 0.0)
+        prob.fsE[:] = good
+        for ps in parts:
+            loc = ps.prob
+            loc.fsE[:] = good[:, ps.part.global_ids()]
+            d = [loc.starE, loc.fsE, loc.starA, loc.srcA, loc.fsA, loc.omega]
+            assert lib().edge_b200_upload_element_data(ps.solver._h, *[ptr(x) for x in d]) == 0
+            assert lib().edge_b200_step_form(ps.solver._h) == 1
+        orc.d = prob.oracle_dict()
+        orc.step(3)
+        steps(3, t)
+    finally:
+        for ps in parts:
+            ps.close()
