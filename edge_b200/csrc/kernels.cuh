@@ -243,8 +243,12 @@ __device__ __forceinline__ void cpAsyncWait() {
 }
 
 // cooperative copy of the rows [R][GB] of quantity row q (of nRows per element) of element e into
-// the tile rows (q, eo * R + row) with stride S, consecutive lanes moving consecutive 16-byte chunks
-template <typename T, int R, int GB, int S>
+// the tile rows (q, eo * R + row) with stride S, consecutive lanes moving consecutive 16-byte chunks.
+// FLAT: rows without padding take one offset for the whole block (no row and column to keep per chunk).
+// The weak-form kernels with attenuation gain by it (LTS at order 4 with 8 runs: 1.63 against 2.01 ms a
+// cycle); the elastic ones lose up to 2% (order 5, FP64, 4,374 elements: 91.9 against 89.8 us a step) and keep
+// rows and columns
+template <typename T, int R, int GB, int S, bool FLAT = false>
 __device__ __forceinline__ void copyRows(T *tile, const T *base, int64_t e, int nRows, int q, int eo, int r) {
   constexpr int W = 16 / int(sizeof(T)), CPRB = GB / W;
   const T *blk = base + (e * nRows + q) * int64_t(R * GB);
@@ -252,8 +256,7 @@ __device__ __forceinline__ void copyRows(T *tile, const T *base, int64_t e, int 
 #pragma unroll
   for (int it = 0; it < CPRB; it++) {
     const int k = it * R + r;
-    if constexpr (S == GB) {
-      // rows without padding: one offset for the whole block (no row and column to keep per chunk)
+    if constexpr (FLAT && S == GB) {
       cpAsync16(dst + k * W, blk + k * W);
     } else {
       const int row = k / CPRB, col = k % CPRB;
@@ -265,15 +268,15 @@ __device__ __forceinline__ void copyRows(T *tile, const T *base, int64_t e, int 
 // cooperative copy of the DOF rows [R][GB] of quantity q of an element into the tile rows
 // (q, eo * R + row) with stride S: warp q moves its quantity's rows, consecutive lanes consecutive
 // 16-byte chunks
-template <typename T, int R, int GB, int S>
+template <typename T, int R, int GB, int S, bool FLAT = false>
 __device__ __forceinline__ void copyDofRows(T *tile, const T *dofsE, int64_t e, int q, int eo, int r) {
-  copyRows<T, R, GB, S>(tile, dofsE, e, 9, q, eo, r);
+  copyRows<T, R, GB, S, FLAT>(tile, dofsE, e, 9, q, eo, r);
 }
 
 // the reverse for results: tile rows (q, eo * R + row), stride S -> the [R][G] rows of row block
 // blk in global memory, consecutive lanes storing consecutive 16-byte chunks (the caller orders the
 // tile rows before, e.g. with __syncwarp when warp q wrote them)
-template <typename T, int R, int G, int S>
+template <typename T, int R, int G, int S, bool FLAT = false>
 __device__ __forceinline__ void storeRowsCoalesced(const T *tile, T *blk, int q, int eo, int r) {
   constexpr int W = 16 / int(sizeof(T)), CPR = G / W;
   const T *src = tile + (q * 32 + eo * R) * S;
@@ -281,11 +284,11 @@ __device__ __forceinline__ void storeRowsCoalesced(const T *tile, T *blk, int q,
   for (int it = 0; it < CPR; it++) {
     const int k = it * R + r;
     const int row = k / CPR, col = k % CPR;
-    const int from = S == G ? k * W : row * S + col * W;
+    const int from = FLAT && S == G ? k * W : row * S + col * W, to = FLAT ? k * W : row * G + col * W;
     if constexpr (sizeof(T) == 4)
-      *reinterpret_cast<float4 *>(blk + k * W) = *reinterpret_cast<const float4 *>(src + from);
+      *reinterpret_cast<float4 *>(blk + to) = *reinterpret_cast<const float4 *>(src + from);
     else
-      *reinterpret_cast<double2 *>(blk + k * W) = *reinterpret_cast<const double2 *>(src + from);
+      *reinterpret_cast<double2 *>(blk + to) = *reinterpret_cast<const double2 *>(src + from);
   }
 }
 
@@ -992,7 +995,7 @@ __device__ __forceinline__ void localFace(const StepArgs<T> &a, const T *TI, T *
     if constexpr (!PM) {
       __syncwarp();
       if (valid)
-        storeRowsCoalesced<T, R, G::GF, SF>(S0, a.face + ((e * 4 + FA) * 9 + q) * int64_t(R * G::GF), q, l / R,
+        storeRowsCoalesced<T, R, G::GF, SF, (RM > 0)>(S0, a.face + ((e * 4 + FA) * 9 + q) * int64_t(R * G::GF), q, l / R,
                                             l % R);
     }
     if constexpr (PM && LTS == 2) {
@@ -1057,7 +1060,7 @@ __device__ __forceinline__ void localFace(const StepArgs<T> &a, const T *TI, T *
     faceMix2<T, F, SF, G::GF>(S0, l, fr, fr1, s, tRow);
     __syncwarp();
     if (ty != FT_OUTFLOW)
-      storeRowsCoalesced<T, R, G::GF, SF>(tile, a.face + ((e * 4 + FA) * 9 + q) * int64_t(R * G::GF), q, l / R,
+      storeRowsCoalesced<T, R, G::GF, SF, (RM > 0)>(tile, a.face + ((e * 4 + FA) * 9 + q) * int64_t(R * G::GF), q, l / R,
                                           l % R);
     if constexpr (LTS) {
       // the LTS buffers of the (pre-mixed) projection t: its sum over the two steps of a pair for a
@@ -1187,7 +1190,7 @@ __device__ __forceinline__ void facesSplit(const StepArgs<T> &a, const T *TI, T 
     for (int i = F; i < G::GF; i++) p[i] = T(0);
     __syncwarp();
     if (valid)
-      storeRowsCoalesced<T, R, G::GF, SF>(tile, a.face + ((e * 4 + fa) * 9 + row) * int64_t(R * G::GF), row, eo,
+      storeRowsCoalesced<T, R, G::GF, SF, (RM > 0)>(tile, a.face + ((e * 4 + fa) * 9 + row) * int64_t(R * G::GF), row, eo,
                                           r);
   }
   cpAsyncWait<0>();
@@ -1253,12 +1256,12 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
     // the first group's DOF rows (and flux-solver blocks of its first face)
     const int64_t g0 = blockIdx.x;
     if (q < 9 && g0 < nGroups && g0 * E + eo < a.elCount)
-      copyDofRows<T, R, G::GB, SB>(TI, a.dofsE, a.elFirst + g0 * E + eo, q, eo, r);
+      copyDofRows<T, R, G::GB, SB, (RM > 0)>(TI, a.dofsE, a.elFirst + g0 * E + eo, q, eo, r);
     if constexpr (AP) {
       if (q >= 9 && g0 < nGroups && g0 * E + eo < a.elCount)
 #pragma unroll
         for (int m = 0; m < RM; m++)
-          copyRows<T, R, G::GB, SB>(TIA, a.dofsA, a.elFirst + g0 * E + eo, RM * 6, m * 6 + q - 9, eo, r);
+          copyRows<T, R, G::GB, SB, (RM > 0)>(TIA, a.dofsA, a.elFirst + g0 * E + eo, RM * 6, m * 6 + q - 9, eo, r);
     }
     if constexpr (PM) issueMixFs<T, O, R, RM, 0>(a, fsb, g0, nGroups);
     if constexpr (FL) issueLocalFs<T, O, R, RM, 0>(a, fsl, g0, nGroups);
@@ -1370,7 +1373,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
     if (q < 9) {
       if constexpr (AS) {
         // the DOF rows again (X is free after the recursion; L2-resident since the group start)
-        if (valid) copyDofRows<T, R, G::GB, SB>(X, a.dofsE, e, q, eo, r);
+        if (valid) copyDofRows<T, R, G::GB, SB, (RM > 0)>(X, a.dofsE, e, q, eo, r);
         cpAsyncCommit();
         cpAsyncWait<0>();
         __syncwarp();
@@ -1394,7 +1397,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         // this group's anelastic rows into this warp's XA rows (free after the recursion)
         if (valid)
 #pragma unroll
-          for (int m = 0; m < RM; m++) copyRows<T, R, G::GB, SB>(XA, a.dofsA, e, RM * 6, m * 6 + q - 9, eo, r);
+          for (int m = 0; m < RM; m++) copyRows<T, R, G::GB, SB, (RM > 0)>(XA, a.dofsA, e, RM * 6, m * 6 + q - 9, eo, r);
         cpAsyncCommit();
       }
 #pragma unroll
@@ -1450,13 +1453,13 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         for (int n = B; n < G::GB; n++) p[n] = T(0);
         __syncwarp();
         if (valid)
-          storeRowsCoalesced<T, R, G::GB, SB>(TI, a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q, eo, r);
+          storeRowsCoalesced<T, R, G::GB, SB, (RM > 0)>(TI, a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q, eo, r);
         if constexpr (AS) {
           // the next group's DOF rows into this warp's TI rows
           __syncwarp();
           const int64_t gn = g + gridDim.x;
           if (gn < nGroups && gn * E + eo < a.elCount)
-            copyDofRows<T, R, G::GB, SB>(TI, a.dofsE, a.elFirst + gn * E + eo, q, eo, r);
+            copyDofRows<T, R, G::GB, SB, (RM > 0)>(TI, a.dofsE, a.elFirst + gn * E + eo, q, eo, r);
         }
       }
       if constexpr (AS) cpAsyncCommit();
@@ -1501,7 +1504,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         if (gn < nGroups && gn * E + eo < a.elCount)
 #pragma unroll
           for (int m = 0; m < RM; m++)
-            copyRows<T, R, G::GB, SB>(TIA, a.dofsA, a.elFirst + gn * E + eo, RM * 6, m * 6 + q - 9, eo, r);
+            copyRows<T, R, G::GB, SB, (RM > 0)>(TIA, a.dofsA, a.elFirst + gn * E + eo, RM * 6, m * 6 + q - 9, eo, r);
         cpAsyncCommit();
       }
     }
@@ -1569,7 +1572,7 @@ struct NeighSlots {
       const int64_t e = a.elFirst + g * E + eo;
 #pragma unroll
       for (int m = 0; m < RM; m++)
-        copyRows<T, R, G::GB, G::SB>(dofATile(base), a.dofsA, e, RM * 6, m * 6 + q - 9, eo, r);
+        copyRows<T, R, G::GB, G::SB, (RM > 0)>(dofATile(base), a.dofsA, e, RM * 6, m * 6 + q - 9, eo, r);
     }
   }
 
@@ -1823,7 +1826,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, Geo<T, O, R, RM>::minCta
         for (int n = B; n < G::GB; n++) p[n] = T(0);
         __syncwarp();
         if (valid)
-          storeRowsCoalesced<T, R, G::GB, G::SB>(NS::dofTile(smem), a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q,
+          storeRowsCoalesced<T, R, G::GB, G::SB, (RM > 0)>(NS::dofTile(smem), a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q,
                                                  eo, r);
         __syncwarp();
       }

@@ -370,7 +370,7 @@ __device__ __forceinline__ void rowsIn(T *tile, const T *dofs, int64_t e0, int n
       if (eo < nv) cpAsync16(tile + (q * 32 + eo) * S + c * G::W, dofs + ((e0 + eo) * NR + q) * G::GB + c * G::W);
     }
   } else {
-    if (l / R < nv) copyRows<T, R, G::GB, S>(tile, dofs, e0 + l / R, NR, q, l / R, l % R);
+    if (l / R < nv) copyRows<T, R, G::GB, S, true>(tile, dofs, e0 + l / R, NR, q, l / R, l % R);
   }
 }
 template <typename T, int O, int R, int S, int NR = 9>
@@ -387,7 +387,7 @@ __device__ __forceinline__ void rowsOut(const T *tile, T *dofs, int64_t e0, int 
     }
   } else {
     if (l / R < nv)
-      storeRowsCoalesced<T, R, G::GB, S>(tile, dofs + ((e0 + l / R) * NR + q) * int64_t(R * G::GB), q, l / R, l % R);
+      storeRowsCoalesced<T, R, G::GB, S, true>(tile, dofs + ((e0 + l / R) * NR + q) * int64_t(R * G::GB), q, l / R, l % R);
   }
 }
 
