@@ -244,11 +244,17 @@ struct edge_b200_ctx {
   // neighbours ([nEl][4][3][R][GF], two of them, alternating with the steps: outCur holds the last
   // written) and those they keep. Without halo parts, the steps of one multi-step call are fused:
   // each step's surface integrals run in the next step's kernel, and the last one's on their own at
-  // the end of the call (flush), so between calls nothing is pending
+  // the end of the call (flush), so between calls nothing is pending. Configurations with
+  // KernelSet::fuseWeak fuse the neighbour steps of the weak form the same way, their projections
+  // alternating with a second face buffer (faceAlt, allocated for a context that needs it; without
+  // memory for it, unfused)
   int outCur = 0;
   bool pending = false, fusedOn = true;
+  DevBuf faceAlt;
+  bool altRefused = false;
+  bool fuses() const { return fusedOn && (strong() || faceAlt.p); }
   char *faceThird(int i) const { return static_cast<char *>(face) + i * (faceCount() / 3 * realSize); }
-  void *outBuf(int i) const { return faceThird(i); }
+  void *outBuf(int i) const { return strong() ? faceThird(i) : i && faceAlt.p ? faceAlt.p : face; }
   // the face that reads each face slot: parts turn halo rows of the other form (kFaceUnpack)
   DevBuf readers;
   bool readersStale = true;
@@ -540,7 +546,13 @@ struct edge_b200_ctx {
   // what a GTS step of this context needs built
   cudaError_t ensureGts() {
     cudaError_t e = ensureStep();
-    return e || strong() ? e : ensureFsLR();
+    if (e || strong()) return e;
+    if (ks->fuseWeak() && fusedOn && nOwned == nEl && !faceAlt.p && !altRefused)
+      if (faceAlt.fit(faceCount() * realSize)) {
+        cudaGetLastError();
+        altRefused = true;
+      }
+    return ensureFsLR();
   }
   // counts the changes of what a captured graph of this context's steps holds (a batch compares it
   // with its value at the capture): element data and mesh, with them the step form and the buffers it
@@ -548,7 +560,7 @@ struct edge_b200_ctx {
   int64_t stepGen = 0;
   void dataChanged() {
     fsLRStale = stepStale = true;
-    stepRejected = false;
+    stepRejected = altRefused = false;
     stepGen++;
     dataGen = data->gen;
   }
@@ -570,11 +582,9 @@ struct edge_b200_ctx {
     if (strong() && !weak) {
       a.fac = fac;
       a.gath = gath;
-      a.face = outBuf(outCur);
       a.wOwn = faceThird(2);
-    } else {
-      a.face = face;
     }
+    a.face = weak ? face : outBuf(outCur);
     a.starE = data->starE;
     a.starA = data->starA;
     a.srcA = data->srcA;
@@ -1027,9 +1037,9 @@ static int runSteps(edge_b200_ctx *ctx, double t, double dt, int n_steps, int ph
   ctx->lastLts = false;
   cudaStream_t s = ctx->stream;
   EDGE_CUDA(ctx->ensureGts(), "step coefficients");
-  // whole strong-form steps without halo parts fold each step's surface integrals into the next
-  // step's kernel; the split phases run them on their own
-  const bool fused = phases == 3 && ctx->fusedOn && ctx->strong() && ctx->nOwned == ctx->nEl;
+  // whole steps without halo parts fold each step's surface integrals (strong form) or neighbour step
+  // (weak form, fuseWeak) into the next step's kernel; the split phases run them on their own
+  const bool fused = phases == 3 && ctx->fuses() && ctx->nOwned == ctx->nEl;
   if (!fused) EDGE_CUDA(ctx->flush(), "pending neighbour step");
   // receiver samples of every step (Receivers::getRecvTimeRel, io/Receivers.cpp:235-248)
   std::vector<int> stepFirst(n_steps + 1, 0);
@@ -1196,7 +1206,7 @@ static int packFaces(edge_b200_ctx *ctx, int n, const int32_t *slots, void *buf,
   if (ctx->meshSet && ctx->dataSet) EDGE_CUDA(ctx->ensureGts(), "step coefficients");
   const bool st = ctx->strong();
   const int64_t stride16 = edge_b200_face_block_bytes(ctx) / 16, nSlots = ctx->nEl * 4;
-  uint4 *face = static_cast<uint4 *>(st ? ctx->outBuf(ctx->outCur) : ctx->face), *blocks = static_cast<uint4 *>(buf);
+  uint4 *face = static_cast<uint4 *>(ctx->outBuf(ctx->outCur)), *blocks = static_cast<uint4 *>(buf);
   cudaStream_t s = ctx->stream;
   if (pack) {
     const int64_t total = (int64_t)n * (st ? stride16 / 3 : stride16);
@@ -1620,9 +1630,8 @@ struct edge_b200_batch {
     dfree(activeDev);
   }
   // contexts whose GTS steps fold each step's surface integrals into the next step's kernel (as
-  // edge_b200_step does): within a call their steps alternate between the two buffers of
-  // characteristics
-  static bool fused(const edge_b200_ctx *c) { return c->fusedOn && c->strong(); }
+  // edge_b200_step does): within a call their steps alternate between the two buffers
+  static bool fused(const edge_b200_ctx *c) { return c->fuses(); }
   // one GTS step of context k on its stream, its sources at t0 + tOff + steps[k] * dt. kind 0: a
   // call's first step (fused contexts: nothing pending, characteristics out to buffer 1); 1: fused,
   // pending ones in buffer 1, out to buffer 0; 2: in buffer 0, out to buffer 1. Other contexts take

@@ -71,6 +71,11 @@ class KernelSetImpl final : public KernelSet {
       return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occLocal_, kLocal<T, O, R, RM, 0>, G::NT, smemLocal())))
       return e;
+    if constexpr (G::fuseWeak) {
+      if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smemLocal())))
+        return e;
+    }
     if constexpr (viscStrong) {
       using V = VGeo<T, O, R, RM>;
       if ((e = cudaFuncSetAttribute(kStepVisc<T, O, R, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V::smem)))
@@ -159,6 +164,12 @@ class KernelSetImpl final : public KernelSet {
         return cudaGetLastError();
       }
     }
+    if constexpr (G::fuseWeak) {
+      if (a.faceIn) {
+        kLocal<T, O, R, RM, 0, true><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
+        return cudaGetLastError();
+      }
+    }
     kLocal<T, O, R, RM, 0><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
     return cudaGetLastError();
   }
@@ -198,6 +209,7 @@ class KernelSetImpl final : public KernelSet {
   }
   bool ltsSupported() const override { return G::ltsOk; }
   bool premix() const override { return G::premix; }
+  bool fuseWeak() const override { return G::fuseWeak; }
   int fsPairStride() const override { return G::FSP; }
   cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) override {
     if (a.elCount < 1) return cudaSuccess;

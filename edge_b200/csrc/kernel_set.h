@@ -28,7 +28,7 @@ struct StepArgsRaw {
   // padded to 16 bytes: [nEl][4][2][fsPairStride()] (premix)
   const void *fsLR = nullptr;
   // strong-form GTS steps (StepArgs): coefficients (null: the weak-form kernels), gather table, own
-  // characteristics, and the characteristics of the previous step that are still pending
+  // characteristics; in both forms what the previous step wrote to face and is still pending
   const void *fac = nullptr;
   const uint32_t *gath = nullptr;
   void *wOwn = nullptr;
@@ -41,8 +41,8 @@ class KernelSet {
  public:
   virtual ~KernelSet() {}
   virtual cudaError_t init(int device) = 0;  // sets smem attributes, sizes the persistent grids
-  // GTS local step: in strong form when a.fac is given (the pending surface integrals of a.faceIn
-  // first), else in weak form
+  // GTS local step: in strong form when a.fac is given, else in weak form; what a.faceIn holds of the
+  // previous step (weak form: with fuseWeak only) is added first
   virtual cudaError_t local(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the configuration has the strong-form step (step.cuh), whose closing half neigh runs when a.fac
   // is given
@@ -56,6 +56,8 @@ class KernelSet {
   virtual bool ltsSupported() const = 0;
   // GTS face projections leave the local kernel mixed with the reader's flux solver (fsLR)
   virtual bool premix() const = 0;
+  // weak-form steps take the pending neighbour step of a.faceIn into the next local step
+  virtual bool fuseWeak() const = 0;
   virtual int fsPairStride() const = 0;
   virtual cudaError_t neigh(const StepArgsRaw &a, cudaStream_t s) = 0;
   // the neighbour step over the buffers the LTS local kernels wrote (pre-mixed where those

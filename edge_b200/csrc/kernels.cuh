@@ -59,11 +59,12 @@ struct StepArgs {
   // strong-form GTS steps (step.cuh): the coefficients of the elements, null for the
   // kernels of this file; per face the packed (neighbour * 4 + its face) * 4 + orientation or
   // 0xffffffff; the elements' own characteristics; face then holds those they
-  // write for their neighbours, and faceIn the previous step's, still to be added to the DOF rows,
-  // or null when none are pending
+  // write for their neighbours
   const T *fac;
   const uint32_t *gath;
   T *wOwn;
+  // fused GTS steps: what the previous step wrote to face (characteristics, or pre-mixed projections in
+  // weak form), still to be added to the DOF rows, or null when nothing is pending
   const T *faceIn;
   // GTS local step with a time step per element group (g = 0 .. of the launch range: E elements
   // each) instead of dt, or null: several simulations merged into one context step together
@@ -334,6 +335,11 @@ struct Geo {
   static constexpr int FSP = padGlobal<T>(81);  // a 9x9 block padded to 16 bytes
   static constexpr size_t premixBytes = size_t(2) * E * 2 * FSP * sizeof(T);
   static constexpr bool premix = RM == 0 && asyncLocal && smemLocal + premixBytes <= localBudget;
+  // weak-form steps fold the neighbour step into the next local kernel (kLocal<..., FUSED>) where that
+  // was faster on 3,000 to 83,000 elements: in FP32 at orders 3 to 5 (1.03 with one run, 1.07 to 1.12 with 8
+  // and 16), not at order 6 (1.01 with 16 runs, 0.98 with 8), order 2 (0.98) or in FP64 (0.89 at order 2,
+  // 0.97 at order 3, 0.99 at order 4; receivers take 3% more off, as they gather what is pending too)
+  static constexpr bool fuseWeak = premix && sizeof(T) == 4 && O >= 3 && O <= 5;
   // configurations that mix in the neighbour kernel (attenuation among them): the local flux-solver
   // blocks fsE[0] (and fsA[0]) of every face arrive one face ahead by cp.async into two buffers
   // [E][NFL] of doubles behind the face tile, where they fit
@@ -958,6 +964,45 @@ __device__ __forceinline__ int neighOri(const FaceMeta &m) {
   return kFacePerm[O - 2][m.src[FA] & 3][FA][m.vert(FA)];
 }
 
+// the neighbour flux of face FA through pre-mixed projections read straight from global memory
+// (this warp's quantity row, this lane's run): the arithmetic of the neighbour kernel's
+// neighApplyMixed, for kernels that fold a pending neighbour step into their DOF rows
+template <typename T, int O, int R, int RM, int FA>
+__device__ __forceinline__ void neighFluxFace(const T *faceIn, const FaceMeta &m, int64_t e, int q, int r,
+                                              bool valid, T *acc) {
+  using G = Geo<T, O, R, RM>;
+  constexpr int F = G::F;
+  const int ty = m.type(FA);
+  if (!valid || ty == FT_OUTFLOW || q >= 9) return;
+  const int64_t src = ty == FT_INNER ? int64_t(m.src[FA]) : e * 4 + FA;
+  T x[F];
+  ldRowG<T, F>(gRow<T, R, G::GF>(faceIn, src, 9, q, r), x, true);
+  if (ty == FT_INNER) {
+    T o[F];
+#pragma unroll
+    for (int j = 0; j < F; j++) o[j] = T(0);
+    const int v = neighOri<O, FA>(m);
+    if (v == 0)
+      OriMul<O, 0>::template run<T>(x, o);
+    else if (v == 1)
+      OriMul<O, 1>::template run<T>(x, o);
+    else
+      OriMul<O, 2>::template run<T>(x, o);
+    FluxTMul<O, FA>::template run<T>(o, acc);
+  } else {
+    FluxTMul<O, FA>::template run<T>(x, acc);
+  }
+}
+template <typename T, int O, int R, int RM>
+__device__ __forceinline__ void neighFluxDirect(const StepArgs<T> &a, const T *faceIn, int64_t e, int q, int r,
+                                                bool valid, T *acc) {
+  FaceMeta m;
+  m.load(a, e, valid);
+  neighFluxFace<T, O, R, RM, 0>(faceIn, m, e, q, r, valid, acc);
+  neighFluxFace<T, O, R, RM, 1>(faceIn, m, e, q, r, valid, acc);
+  neighFluxFace<T, O, R, RM, 2>(faceIn, m, e, q, r, valid, acc);
+  neighFluxFace<T, O, R, RM, 3>(faceIn, m, e, q, r, valid, acc);
+}
 
 // ------------------------------------------------------------------------------------------------
 // local step: CK, volume, local surface, face projections (AderDg::local, AderDg.hpp:338-534)
@@ -1205,7 +1250,10 @@ __device__ __forceinline__ void facesSplit(const StepArgs<T> &a, const T *TI, T 
 
 // LTS as in localFace; mode 2 keeps the half-step integral in one more tile (one CTA per SM), mode
 // 1 runs on the elements of a time group without a smaller neighbour
-template <typename T, int O, int R, int RM, int LTS>
+// FUSED (GTS, Geo::fuseWeak): the previous step's neighbour fluxes (a.faceIn) are added to each group's
+// DOF rows first, and the completed rows stored back: a pass over the DOFs and a launch less per step
+// than kNeigh after it (order 5, 16 runs, FP32, 48,000 elements: 2.30 against 2.50 ms a step)
+template <typename T, int O, int R, int RM, int LTS, bool FUSED = false>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O, R, RM>::minCtasLocal)
     kLocal(StepArgs<T> a) {
   using G = Geo<T, O, R, RM>;
@@ -1221,6 +1269,7 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
   // alternate between a separate face tile (even faces) and X (odd faces): one barrier per face
   // instead of two (the last face keeps both)
   constexpr bool AS = G::asyncLocal;
+  static_assert(!FUSED || (AS && G::fuseWeak && LTS == 0), "fused weak-form steps");
   T *TI = G::tiSmem ? X + G::nX : X;
   T *TIA = G::tiSmem ? XA + G::nXA : XA;
   T *S0 = AS ? TIA + G::nTIA : (G::tiSmem ? X : X + G::nX);
@@ -1291,6 +1340,18 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT, LTS == 2 ? 1 : Geo<T, O,
         else
 #pragma unroll
           for (int n = 0; n < B; n++) v[n] = T(0);
+        if constexpr (FUSED) {
+          neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
+          // the completed rows back to the DOFs (the volume integral reads them again)
+          T *p = rowPtr<T, SB>(X, q, l);
+          stRow<T, B>(p, v);
+#pragma unroll
+          for (int n = B; n < G::GB; n++) p[n] = T(0);
+          __syncwarp();
+          if (valid)
+            storeRowsCoalesced<T, R, G::GB, SB>(X, a.dofsE + (e * 9 + q) * int64_t(R * G::GB), q, eo, r);
+          __syncwarp();
+        }
         stRow<T, B>(rowPtr<T, SB>(X, q, l), v);
       } else {
         ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, ev, 9, q, r), v, valid);
@@ -1944,8 +2005,8 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
   T zero[B];
 #pragma unroll
   for (int n = 0; n < B; n++) zero[n] = T(0);
-  // pending characteristics of a strong-form step complete the rows first (their tile lies over X and
-  // TI, which are written only after every warp has read it)
+  // what is pending of the previous step completes the rows first (the tile of a strong-form step's
+  // characteristics lies over X and TI, which are written only after every warp has read it)
   T v[B];
   if (q < 9) {
     ldRowG<T, B>(gRow<T, R, G::GB>(a.dofsE, ev, 9, q, r), v, valid);
@@ -1953,7 +2014,9 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
 #pragma unroll
     for (int n = 0; n < B; n++) v[n] = T(0);
   }
-  if (a.faceIn) {
+  if (a.faceIn && !a.fac) {
+    if constexpr (G::fuseWeak) neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
+  } else if (a.faceIn) {
     static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
     for (int t = q; t < 12; t += G::NW) liftRow<T, O, R, false>(a, a.faceIn, X, t, l, ev, r, valid);
     __syncthreads();

@@ -238,3 +238,39 @@ def test_godunov_solvers_of_strong_contrasts_take_the_strong_form(order, rm):
     orc.step(4)
     assert rel_l2(s.download_dofs()[0], orc.state["dofsE"]) < 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("order,runs,rm,prec,full_rank,fuses", [
+    (5, 16, 0, 32, True, True), (4, 8, 0, 32, True, True), (3, 1, 0, 32, True, True), (3, 4, 0, 32, True, True),
+    (6, 16, 0, 32, True, False), (4, 1, 0, 64, True, False), (5, 1, 0, 64, True, False), (5, 4, 0, 32, True, False), (4, 8, 3, 32, True, False),
+    (5, 16, 0, 32, False, True), (5, 1, 0, 64, False, True), (4, 8, 3, 32, False, True)])
+def test_steps_fuse_in_both_forms(order, runs, rm, prec, full_rank, fuses):
+    """Multi-step calls fold each step's surface integrals into the next step's kernel in the strong form,
+    and the neighbour steps of weak-form contexts at orders 3 to 5 in FP32 with pre-mixed projections: one
+    closing launch a call instead of one a step, the same DOFs and receiver samples as without."""
+    prob = small_problem(n=3, order=order, runs=runs, rm=rm, jitter=0.15, n_steps=6, source="random",
+                         layers=[3000.0, 6000.0], lognormal_sigma=0.2)
+    if full_rank:
+        prob = _penalised(prob)
+    e0, a0 = random_dofs(prob, seed=3)
+    a, b = Solver(prob, precision=prec), Solver(prob, precision=prec)
+    assert lib().edge_b200_set_fused(b._h, 0) == 0
+    for x in (a, b):
+        assert lib().edge_b200_step_form(x._h) == (0 if full_rank else 1)
+        x.upload_dofs(e0, a0)
+    for k in (1, 3, 2):  # calls of one and of several steps
+        a.step(k)
+        b.step(k)
+        assert b.launches() - a.launches() == (k - 1 if fuses else 0)
+    for x, y in zip(a.download_dofs(), b.download_dofs()):
+        np.testing.assert_array_equal(x, y)
+    ra, rb = a.receivers(), b.receivers()
+    k = int(ra[2][0])
+    assert k > 0
+    np.testing.assert_array_equal(ra[2], rb[2])
+    np.testing.assert_array_equal(ra[0][:, :k], rb[0][:, :k])
+    orc = OracleRun(prob, e0, a0)
+    orc.step(6)
+    assert rel_l2(a.download_dofs()[0], orc.state["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
+    a.close()
+    b.close()
