@@ -1551,12 +1551,14 @@ int64_t edge_b200_last_launches(const edge_b200_ctx *ctx) { return ctx ? ctx->la
 
 int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]) {
   if (!ctx || !info) return EDGE_B200_EINVAL;
-  info[5] = (ctx->fusedOn && ctx->ks->premix() && ctx->nOwned == ctx->nEl) ? 1 : 0;
+  // the form of the steps as far as known (before the data are set, that of Godunov solvers)
+  const bool st = ctx->ks->strongSupported() && !ctx->stepRejected;
   info[0] = ctx->ks->elementsPerCta();
-  info[1] = ctx->ks->premix() ? (ctx->ks->strongSupported() && !ctx->stepRejected ? 2 : 1) : 0;
+  info[1] = ctx->ks->premix() ? (st ? 2 : 1) : 0;
   info[2] = ctx->ks->fsPairStride();
-  info[3] = ctx->ks->ctasLocal();
-  info[4] = ctx->ks->ctasNeigh();
+  info[3] = ctx->ks->ctasLocal(st);
+  info[4] = ctx->ks->ctasNeigh(st);
+  info[5] = ctx->ks->premix() && ctx->fusedOn && (st || ctx->ks->fuseWeak()) && ctx->nOwned == ctx->nEl ? 1 : 0;
   return EDGE_B200_OK;
 }
 
@@ -1861,11 +1863,17 @@ int edge_b200_autotune(edge_b200_ctx *ctx, double dt, int32_t caps[2]) {
   KernelSet *ks = ctx->ks;
   ks->setGridCaps(0, 0);
   const int64_t groups = (ctx->nOwned + ks->elementsPerCta() - 1) / ks->elementsPerCta();
-  const int defL = ks->ctasLocal(), defN = ks->ctasNeigh();
+  const int defL = ks->ctasLocal(ctx->strong()), defN = ks->ctasNeigh(ctx->strong());
   cudaEvent_t ev[2];
   EDGE_CUDA(cudaEventCreate(&ev[0]), "autotune");
   EDGE_CUDA(cudaEventCreate(&ev[1]), "autotune");
   StepArgsRaw a = ctx->args(dt);
+  StepArgsRaw aLocal = a;
+  if (ctx->fuses() && ctx->nOwned == ctx->nEl) {
+    // the kernel of a multi-step call: the previous step's rows in (any will do), this step's out
+    aLocal.faceIn = ctx->outBuf(ctx->outCur);
+    aLocal.face = ctx->outBuf(ctx->outCur ^ 1);
+  }
   int best[2] = {0, 0};
   cudaError_t err = cudaSuccess;
   for (int kind = 0; kind < 2 && !err; kind++) {
@@ -1882,7 +1890,7 @@ int edge_b200_autotune(edge_b200_ctx *ctx, double dt, int32_t caps[2]) {
       float ms = 1e30f;
       for (int rep = 0; rep < 4 && !err; rep++) {
         if ((err = cudaEventRecord(ev[0], s))) break;
-        err = kind == 0 ? ks->local(a, s) : ks->neigh(a, s);
+        err = kind == 0 ? ks->local(aLocal, s) : ks->neigh(a, s);
         if (!err) err = cudaEventRecord(ev[1], s);
         if (!err) err = cudaEventSynchronize(ev[1]);
         float t = 0;

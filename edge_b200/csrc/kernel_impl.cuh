@@ -135,8 +135,12 @@ class KernelSetImpl final : public KernelSet {
     return cudaSuccess;
   }
   int elementsPerCta() const override { return G::E; }
-  int ctasLocal() const override { return capLocal_ > 0 ? capLocal_ : numSms_ * occLocal_; }
-  int ctasNeigh() const override { return capNeigh_ > 0 ? capNeigh_ : numSms_ * occNeigh_; }
+  int ctasLocal(bool strong) const override {
+    return capLocal_ > 0 ? capLocal_ : numSms_ * (strong ? occStep_ : occLocal_);
+  }
+  int ctasNeigh(bool strong) const override {
+    return capNeigh_ > 0 ? capNeigh_ : numSms_ * (strong ? occLift_ : occNeigh_);
+  }
   void setGridCaps(int local, int neigh) override {
     capLocal_ = local;
     capNeigh_ = neigh;
@@ -153,24 +157,24 @@ class KernelSetImpl final : public KernelSet {
       using V = VGeo<T, O, R, RM>;
       if (a.fac) {
         kStepVisc<T, O, R, RM>
-            <<<grid(a.elCount, capLocal_ > 0 ? capLocal_ : numSms_ * occStep_), V::NT, V::smem, s>>>(cast(a));
+            <<<grid(a.elCount, ctasLocal(true)), V::NT, V::smem, s>>>(cast(a));
         return cudaGetLastError();
       }
     }
     if constexpr (RM == 0) {
       using S = SGeo<T, O, R>;
       if (a.fac) {
-        kStep<T, O, R><<<grid(a.elCount, capLocal_ > 0 ? capLocal_ : numSms_ * occStep_), S::NT, S::smem, s>>>(cast(a));
+        kStep<T, O, R><<<grid(a.elCount, ctasLocal(true)), S::NT, S::smem, s>>>(cast(a));
         return cudaGetLastError();
       }
     }
     if constexpr (G::fuseWeak) {
       if (a.faceIn) {
-        kLocal<T, O, R, RM, 0, true><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
+        kLocal<T, O, R, RM, 0, true><<<grid(a.elCount, ctasLocal(false)), G::NT, smemLocal(), s>>>(cast(a));
         return cudaGetLastError();
       }
     }
-    kLocal<T, O, R, RM, 0><<<grid(a.elCount, ctasLocal()), G::NT, smemLocal(), s>>>(cast(a));
+    kLocal<T, O, R, RM, 0><<<grid(a.elCount, ctasLocal(false)), G::NT, smemLocal(), s>>>(cast(a));
     return cudaGetLastError();
   }
   bool strongSupported() const override { return RM == 0 || viscStrong; }
@@ -217,18 +221,18 @@ class KernelSetImpl final : public KernelSet {
       using V = VGeo<T, O, R, RM>;
       if (a.fac) {
         kLiftVisc<T, O, R, RM>
-            <<<grid(a.elCount, capNeigh_ > 0 ? capNeigh_ : numSms_ * occLift_), V::NT, V::smemLift, s>>>(cast(a));
+            <<<grid(a.elCount, ctasNeigh(true)), V::NT, V::smemLift, s>>>(cast(a));
         return cudaGetLastError();
       }
     }
     if constexpr (RM == 0) {
       using S = SGeo<T, O, R>;
       if (a.fac) {
-        kLift<T, O, R><<<grid(a.elCount, capNeigh_ > 0 ? capNeigh_ : numSms_ * occLift_), S::NT, S::smemLift, s>>>(cast(a));
+        kLift<T, O, R><<<grid(a.elCount, ctasNeigh(true)), S::NT, S::smemLift, s>>>(cast(a));
         return cudaGetLastError();
       }
     }
-    kNeigh<T, O, R, RM, G::premix><<<grid(a.elCount, ctasNeigh()), G::NT, smemNeigh(), s>>>(cast(a));
+    kNeigh<T, O, R, RM, G::premix><<<grid(a.elCount, ctasNeigh(false)), G::NT, smemNeigh(), s>>>(cast(a));
     return cudaGetLastError();
   }
   cudaError_t neighLts(const StepArgsRaw &a, cudaStream_t s) override {
@@ -240,7 +244,7 @@ class KernelSetImpl final : public KernelSet {
         return cudaGetLastError();
       }
     }
-    kNeigh<T, O, R, RM, G::premixLts><<<grid(a.elCount, ctasNeigh()), G::NT, smemNeigh(), s>>>(cast(a));
+    kNeigh<T, O, R, RM, G::premixLts><<<grid(a.elCount, ctasNeigh(false)), G::NT, smemNeigh(), s>>>(cast(a));
     return cudaGetLastError();
   }
   cudaError_t recv(const StepArgsRaw &a, const RecvArgs &r, cudaStream_t s) override {

@@ -66,8 +66,9 @@ class KernelSet {
   virtual cudaError_t recv(const StepArgsRaw &a, const RecvArgs &r, cudaStream_t s) = 0;
   virtual cudaError_t sources(void *dofsE, const SrcArgs &sa, cudaStream_t s) = 0;
   virtual int elementsPerCta() const = 0;
-  virtual int ctasLocal() const = 0;
-  virtual int ctasNeigh() const = 0;
+  // persistent grids of the GTS local / neighbour kernels in the strong or the weak form
+  virtual int ctasLocal(bool strong) const = 0;
+  virtual int ctasNeigh(bool strong) const = 0;
   // caps on the persistent grids of the GTS local / neighbour kernels (0: resident CTAs per SM x
   // SMs, the default; a larger cap gives one CTA per element group up to it)
   virtual void setGridCaps(int local, int neigh) = 0;

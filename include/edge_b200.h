@@ -316,23 +316,24 @@ int edge_b200_set_timing(edge_b200_ctx *ctx, int enable);
  * flux, which arrive as three characteristic rows per face from each side) inside the next step's
  * kernel, before its recursion; the receiver kernel does the same for its elements. The last step's
  * surface integrals run on their own before the call returns, so the DOFs are complete between
- * calls. Same arithmetic as the separate kernels: the results are identical. No counterpart in the
- * reference.
+ * calls. Same arithmetic as the separate kernels: the results are identical. Weak-form steps fuse
+ * their neighbour steps the same way in FP32 at orders 3 to 5 with pre-mixed projections (with a second
+ * face buffer; without memory for it they stay separate). No counterpart in the reference.
  * The strong form is taken by every configuration whose rows fit the kernels (all elastic ones; with
  * 3 mechanisms up to order 5 in FP32 and order 4 in FP64) as long as every face's flux solvers, with
  * the element's own flux across the face taken off, act through three waves -- Godunov fluxes of
- * elastic media do; the first GTS step after the mesh or element data changed checks it. Otherwise
- * GTS steps run the weak-form kernels, unfused. */
+ * elastic media do; checked when the mesh and the element data are set. What they leave out of that may
+ * be 1e-13 of the solvers in FP64, 1e-9 in FP32. Otherwise GTS steps run the weak-form kernels. */
 int edge_b200_set_fused(edge_b200_ctx *ctx, int enable);
 int edge_b200_kernel_times(edge_b200_ctx *ctx, double *ms, int64_t *launches);
 /* Launch shape of the context's compiled configuration (no counterpart in the reference, whose
  * kernels run one element per thread team): info[0] elements per CTA, info[3] / info[4] persistent
- * CTAs of the weak-form local / neighbour kernel. info[1], info[2] and info[5] describe the weak-form
- * kernels' buffers: info[1] 1 when face projections leave the local kernel pre-mixed with the reading
- * element's flux solver (per element face the padded pair [2][info[2]] of flux solvers in the
+ * CTAs of the GTS local / neighbour kernel of the context's step form. info[1] and info[2] describe the
+ * weak-form kernels' buffers: info[1] 1 when face projections leave the local kernel pre-mixed with the
+ * reading element's flux solver (per element face the padded pair [2][info[2]] of flux solvers in the
  * configuration's precision), 2 when such a configuration's steps exchange characteristic rows (the
- * strong form) as far as known, info[5] 1 when info[1] > 0 and fused steps are on. edge_b200_step_form tells
- * which form the GTS steps take. */
+ * strong form) as far as known. info[5]: 1 when info[1] > 0 and multi-step calls fuse (edge_b200_set_fused;
+ * contexts with info[1] = 0 fuse when edge_b200_step_form gives 1). */
 int edge_b200_kernel_config(const edge_b200_ctx *ctx, int32_t info[6]);
 /* The form of the context's next GTS step (EDGE_B200_EINVAL before mesh and element data are set):
  * 1 strong, 0 weak (see edge_b200_set_fused). Builds the step's coefficients if they are not built. */

@@ -274,3 +274,30 @@ def test_steps_fuse_in_both_forms(order, runs, rm, prec, full_rank, fuses):
     assert rel_l2(a.download_dofs()[0], orc.state["dofsE"]) < (1e-12 if prec == 64 else 1e-4)
     a.close()
     b.close()
+
+
+# (order, runs, precision), then for the strong and the weak form: CTAs per SM of the local and the
+# neighbour kernel, fused steps
+SHAPES = [((3, 1, 64), (2, 2, 1), (1, 1, 0)), ((4, 1, 64), (1, 2, 1), (1, 1, 0)), ((5, 16, 32), (2, 3, 1), (2, 2, 1)),
+          ((6, 16, 32), (1, 2, 1), (1, 2, 0))]
+
+
+@pytest.mark.parametrize("cfg,strong,weak", SHAPES)
+def test_kernel_config_and_autotuner_know_the_kernels_that_run(cfg, strong, weak):
+    import torch
+    from edge_b200._lib import ptr
+    order, runs, prec = cfg
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    prob = small_problem(n=3, order=order, runs=runs, jitter=0.1, n_steps=1, source=None, n_receivers=0)
+    for p, (local, neigh, fused), form in ((prob, strong, 2), (_penalised(prob), weak, 1)):
+        s = Solver(p, precision=prec)
+        info, caps = np.zeros(6, np.int32), np.zeros(2, np.int32)
+        assert lib().edge_b200_kernel_config(s._h, ptr(info)) == 0
+        assert (info[1], info[3], info[4], info[5]) == (form, local * sms, neigh * sms, fused)
+        s.step(3)
+        assert s.launches() == (4 if fused else 6)
+        assert lib().edge_b200_autotune(s._h, prob.dt, ptr(caps)) == 0
+        groups = -(-p.n_el * runs // 32)
+        for cap, grid in zip(caps, info[3:5]):
+            assert cap in (0, grid // 2) or cap == groups > grid
+        s.close()
