@@ -301,3 +301,57 @@ def test_kernel_config_and_autotuner_know_the_kernels_that_run(cfg, strong, weak
         for cap, grid in zip(caps, info[3:5]):
             assert cap in (0, grid // 2) or cap == groups > grid
         s.close()
+
+
+@pytest.mark.parametrize("order,runs,prec", [(5, 16, 32), (3, 8, 32), (4, 1, 64)])
+def test_lts_in_weak_form_matches(order, runs, prec):
+    """Elastic rate-2 LTS with flux solvers of full rank at one face: the weak-form LTS kernels."""
+    import oracle
+    from test_lts import _grouped, _lts_state
+    prob, gf, flags, rel = _grouped(order=order, n=4, runs=runs, n_receivers=4, source="random", n_steps=30, jitter=0.1)
+    prob = _penalised(prob)
+    e0, _ = random_dofs(prob, seed=9, scale=1e-2)
+    ref = OracleRun(prob, e0.copy())
+    st = _lts_state(prob, e0.copy())
+    oracle.lts_cycles(ref.d, st, gf, 0.0, prob.dt, 2, flags, rel, ref.recv, ref.src)
+    s = Solver(prob, precision=prec)
+    assert lib().edge_b200_step_form(s._h) == 0
+    s.upload_dofs(e0.astype(s.dtype))
+    s.step(2)  # (fused where weak steps fuse: the LTS steps after it use one face buffer)
+    s.upload_dofs(e0.astype(s.dtype))
+    s._chk(lib().edge_b200_rewind_receivers(s._h, prob.receivers["t_first"]), "rewind_receivers")
+    s.set_time_groups(gf)
+    s.t = 0.0
+    s.step_lts(1)
+    s.step_lts(1)
+    tol = 1e-12 if prec == 64 else 1e-4
+    assert rel_l2(s.download_dofs()[0], st["dofsE"]) < tol
+    rb, _, rc = s.receivers()
+    assert np.array_equal(rc, ref.recv["count"])
+    for i, k in enumerate(rc):
+        assert rel_l2(rb[i, :k], ref.recv["buf"][i, :k]) < tol
+    s.close()
+
+
+@pytest.mark.parametrize("prec", [32, 64])
+def test_source_integrals_of_several_blocks_of_steps(prec):
+    """So many sources that a call's series integrals are computed in blocks of four steps."""
+    prob = small_problem(n=2, order=4, runs=8 if prec == 32 else 1, jitter=0.1, n_steps=12, source="random",
+                         n_receivers=0)
+    src, k = prob.sources, -(-30000 // prob.sources["n"])
+    for key in ("el", "run", "scal", "bEval", "t0", "dt", "tsOff", "nPts"):
+        src[key] = np.repeat(src[key], k, axis=0)
+    src["scal"] = src["scal"] / k
+    src["n"] *= k
+    assert 4 <= 131072 // src["n"] < 5
+    e0, _ = prob.zero_dofs()
+    s = Solver(prob, precision=prec)
+    s.upload_dofs(e0)
+    for n in (11, 2, 3):
+        s.step(n)
+    orc = OracleRun(prob, e0.copy())
+    orc.step(16)
+    assert np.abs(orc.state["dofsE"]).max() > 0
+    # a DOF takes k sums a step, each rounded by half a unit: at most 16 * 30,000 * 2^-53, 16 * 3,750 * 2^-24
+    assert rel_l2(s.download_dofs()[0], orc.state["dofsE"]) < 16 * k * 2.0 ** (-53 if prec == 64 else -24)
+    s.close()
