@@ -73,7 +73,9 @@ class KernelSetImpl final : public KernelSet {
       return e;
     if constexpr (G::fuseWeak) {
       if ((e = cudaFuncSetAttribute(kLocal<T, O, R, RM, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smemLocal())))
+                                    (int)smemLocal())) ||
+          (e = cudaFuncSetAttribute(kRecv<T, O, R, RM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smemRecv())))
         return e;
     }
     if constexpr (viscStrong) {
@@ -250,6 +252,12 @@ class KernelSetImpl final : public KernelSet {
   cudaError_t recv(const StepArgsRaw &a, const RecvArgs &r, cudaStream_t s) override {
     const int g = (r.nGrp + G::E - 1) / G::E;
     if (g == 0) return cudaSuccess;
+    if constexpr (G::fuseWeak) {
+      if (a.faceIn && !a.fac) {
+        kRecv<T, O, R, RM, true><<<g, G::NT, smemRecv(), s>>>(cast(a), r);
+        return cudaGetLastError();
+      }
+    }
     kRecv<T, O, R, RM><<<g, G::NT, smemRecv(), s>>>(cast(a), r);
     return cudaGetLastError();
   }

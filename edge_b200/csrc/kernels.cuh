@@ -1984,7 +1984,9 @@ struct FacU;
 template <typename T, int O, int R, typename Z>
 __device__ __forceinline__ void liftApply(const T *wt, const Z &U, int l, T *acc);
 
-template <typename T, int O, int R, int RM>
+// WEAK (Geo::fuseWeak): a weak-form step is pending (in a kernel of its own: beside the characteristics' path
+// it cost every sample of order 3 with 4 runs 1.2 us)
+template <typename T, int O, int R, int RM, bool WEAK = false>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, RecvArgs rv) {
   using G = Geo<T, O, R, RM>;
   constexpr int B = G::B, E = G::E, SB = G::SB;
@@ -2014,8 +2016,8 @@ __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, Rec
 #pragma unroll
     for (int n = 0; n < B; n++) v[n] = T(0);
   }
-  if (a.faceIn && !a.fac) {
-    if constexpr (G::fuseWeak) neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
+  if constexpr (WEAK) {
+    neighFluxDirect<T, O, R, RM>(a, a.faceIn, ev, q, r, valid, v);
   } else if (a.faceIn) {
     static_assert(SGeo<T, O, R>::nWt * sizeof(T) <= G::smemLocal, "tile of the incoming characteristics");
     for (int t = q; t < 12; t += G::NW) liftRow<T, O, R, false>(a, a.faceIn, X, t, l, ev, r, valid);
