@@ -453,15 +453,15 @@ def run_serve(n_req, rate, device, seed=3343, n_check=12):
 
 
 def run_tc_probe(local_ms, n_el, order, runs, device, clock_mhz):
-    """The tensor-core alternative for the local kernel's DG products, measured: tcgen05.mma
+    """The tensor-core alternative for the step kernel's DG products, measured: tcgen05.mma
     (kind::tf32, and kind::f16 with bf16 operands; operands in shared memory, accumulator in tensor
     memory) timed per instruction of 128 x N x K (K = 8 tf32, 16 bf16) for the N the products would
-    have, with one and two issuing CTAs per SM, then the instructions one local step needs in the
+    have, with one and two issuing CTAs per SM, then the instructions one strong-form step needs in the
     tensor formulation -- rows (quantity, element, run) on M in tiles of 128 (the 288 rows of an
     element group in three tiles), output modes on N (padded to 16), input modes x 3 derivative
-    directions (or x 4 faces) on K, each product three times for FP32-level accuracy (split
-    operands: 3xtf32 or 3xbf16) -- at the measured cycles. Only the products: the star and
-    flux-solver mixes, the operand splits, loads, stores and tensor-memory read-back come on top."""
+    directions (or x 3 faces: the mirrored faces 2 and 3 share one product each way) on K, each product
+    three times for FP32-level accuracy (split operands: 3xtf32 or 3xbf16) -- at the measured cycles.
+    Only the products: the star and characteristic mixes, the operand splits, loads, stores and tensor-memory read-back come on top."""
     from edge_b200 import tcprobe
     from edge_b200.host import n_face_modes, n_modes
     errs = {f"{kind}_{n}x{k}x{it}": tcprobe.check(n, k, it, kind=kind)
@@ -486,8 +486,7 @@ def run_tc_probe(local_ms, n_el, order, runs, device, clock_mhz):
     Bm = lambda o: n_modes(o) if o > 0 else 0
     F = n_face_modes(order)
     prods = [("ck%d" % d, pad(Bm(order - d), 16), 3 * Bm(order - d + 1)) for d in range(1, order)]
-    prods += [("volume", pad(Bm(order), 16), 3 * Bm(order - 1)), ("fluxL", pad(4 * F, 16), Bm(order)),
-              ("fluxT", pad(Bm(order), 16), 4 * F)]
+    prods += [("fluxL", pad(3 * F, 16), Bm(order)), ("fluxT", pad(Bm(order), 16), 3 * F)]
     groups_per_sm = n_el * runs / 32 / 148
     tiles, split = 3, 3
 
@@ -867,9 +866,9 @@ def main():
                 "achieved_tflops": flops_launch / (avg_ms / 1e3) / 1e12,
                 "kernel_avg_ms": {names[i]: float(kms[i] / kn[i]) for i in range(4) if kn[i]},
                 "kernel_share": shares}
-    # the local kernel is bound by the FP32 pipe, not HBM: its dense-equivalent flops (the DG
-    # products counted dense; the kernel executes FMAs for the non-zeros only) against the nominal
-    # FP32 CUDA-core peak (SMs x 128 FMA lanes x 2 flops x max SM clock)
+    # the kernel's dense-equivalent flops (the DG products counted dense; it executes FMAs for the
+    # non-zeros only, and is bound by latency rather than by the pipe) against the nominal FP32 CUDA-core
+    # peak (SMs x 128 FMA lanes x 2 flops x max SM clock)
     if prec == 32:
         sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         fp32_peak = sms * 128 * 2 * peak_clock_mhz() * 1e6 / 1e12

@@ -228,13 +228,13 @@ struct edge_b200_ctx {
   int32_t *elFaEl = nullptr;
   uint8_t *fId = nullptr, *vId = nullptr, *faType = nullptr;
   bool meshSet = false, dataSet = false, keepTDofs = false;
-  // flux-solver pairs of the pre-mixed face projections (configurations with KernelSet::premix),
-  // rebuilt before the next GTS step after the mesh or the element data changed
+  // flux-solver pairs of the pre-mixed face projections (configurations with KernelSet::premix), built
+  // before the next weak-form step after the mesh or the element data changed
   DevBuf fsLR;
   bool fsLRStale = true;
-  // strong-form GTS steps (step.cuh): coefficients and gather table, rebuilt before the next GTS step
-  // after the mesh or the element data changed; flux solvers that are not of rank 3 in that form
-  // keep the context on the weak-form kernels until the data change again
+  // strong-form GTS steps (step.cuh): coefficients and gather table, built where the mesh or the element
+  // data are set (a borrower's new data: before its next step); flux solvers that are not of rank 3 in
+  // that form keep the context on the weak-form kernels until the data change again
   void *fac = nullptr;  // fac, gath and stepBad lie behind the face buffer, in its allocation
   uint32_t *gath = nullptr;
   int *stepBad = nullptr;
@@ -573,7 +573,8 @@ struct edge_b200_ctx {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return EDGE_B200_EDEVICE;
   }
-  // weak: for the weak-form kernels (LTS), whatever form the GTS steps take
+  // weak: for the weak-form kernels, whatever form the GTS steps take (LTS with attenuation has no
+  // strong form)
   StepArgsRaw args(double dt, bool weak = false) const {
     StepArgsRaw a;
     a.dofsE = dofsE;

@@ -1,12 +1,12 @@
-"""The characteristic face mix of the local kernel rests on one property of the elastic flux
-solvers: for every face, the element's own flux solver fsE[0] and the one its face reader applies
-(fsE[1] of the neighbour at its face, the element's own for a free surface, none for outflow),
-stacked into an 18 x 9 matrix, have rank 3 -- the three waves (P, S, S) that leave the element
-through the face. The device then mixes each face projection through three characteristic rows
-instead of two 9 x 9 blocks. Checked here on the host-built flux solvers (pinned to the reference's
-Elasticity code in test_host_setup.py) for heterogeneous, layered, jittered meshes with every face
-type, with the oracle's restatement of the factorisation the device builds (column-scaled
-Gram-Schmidt with pivoting, each direction orthogonalised twice)."""
+"""A property of the elastic flux solvers behind the characteristic exchange: for every face, the
+element's own flux solver fsE[0] and the one its face reader applies (fsE[1] of the neighbour at its
+face, the element's own for a free surface, none for outflow), stacked into an 18 x 9 matrix, have
+rank 3 -- the three waves (P, S, S) that leave the element through the face. (The factors that the
+strong-form step builds, with the element's own flux across the face taken off fsE[0], are restated in
+test_strong_form.py.) Checked here on the host-built flux solvers (pinned to the reference's Elasticity
+code in test_host_setup.py) for heterogeneous, layered, jittered meshes with every face type, with the
+oracle's factorisation (column-scaled Gram-Schmidt with pivoting, each direction orthogonalised
+twice)."""
 import numpy as np
 import pytest
 

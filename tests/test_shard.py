@@ -1,7 +1,8 @@
 """Halo partitions (edge_b200.shard): index tables on one process, and multi-rank gloo runs of the
 oracle's local / neighbour work regions with the per-step exchange, against the one-domain run.
 
-The ranks exchange what the device form exchanges: the face rows of the send faces, projected on
+The ranks exchange what the device's weak form exchanges (parts in strong form send characteristics of
+the same rows, tests/test_gpu_halo.py): the face rows of the send faces, projected on
 the face and pre-mixed with the reading element's flux solver (oracle.face_rows_premixed), sent
 after the send elements' local step and before the inner elements' one, and lifted by the
 reader with the face orientation and fluxT. So the partition, the local numbering (send elements
@@ -72,7 +73,7 @@ def _free_port():
 def _rank_main(rank, world, port, order, n_steps, out_dir):
     """One rank: the oracle's local step of the send elements, the pre-mixed face rows of the send
     faces to the peers (gloo), the local step of the inner elements, the neighbour step with the
-    received rows for the ghost faces -- the device form's step order and exchange format."""
+    received rows for the ghost faces -- the device's step order and weak-form exchange format."""
     import torch
 
     import oracle
