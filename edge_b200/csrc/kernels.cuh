@@ -1984,8 +1984,8 @@ struct FacU;
 template <typename T, int O, int R, typename Z>
 __device__ __forceinline__ void liftApply(const T *wt, const Z &U, int l, T *acc);
 
-// WEAK (Geo::fuseWeak): a weak-form step is pending (in a kernel of its own: beside the characteristics' path
-// it cost every sample of order 3 with 4 runs 1.2 us)
+// WEAK (Geo::fuseWeak): a weak-form step is pending; in a kernel of its own, so that the code of the
+// characteristics' path stays as it is without it (no difference in time was measured beyond the noise)
 template <typename T, int O, int R, int RM, bool WEAK = false>
 __global__ void __launch_bounds__(Geo<T, O, R, RM>::NT) kRecv(StepArgs<T> a, RecvArgs rv) {
   using G = Geo<T, O, R, RM>;
